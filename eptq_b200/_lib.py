@@ -10,6 +10,7 @@ from pathlib import Path
 from typing import Optional
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libeptq_b200.so"
+HOST_PATH = LIB_PATH.with_name("_eptq_host.so")
 
 EPTQ_E8, EPTQ_E8D4 = 0, 1
 QUANTIZER_ID = {"e8_lattice": EPTQ_E8, "e8_d4": EPTQ_E8D4}
@@ -96,6 +97,28 @@ def load() -> C.CDLL:
         raise RuntimeError("libeptq_b200.so has an unexpected ABI version")
     _lib = lib
     return lib
+
+
+_host = None
+
+
+def host():
+    """The native host path of module calls (csrc/host/launch.cpp), loaded once."""
+    global _host
+    if _host is None:
+        import importlib.machinery
+        import importlib.util
+
+        import torch  # noqa: F401  (the extension resolves its symbols against torch's libraries)
+        load()
+        if not HOST_PATH.exists():
+            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m eptq_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_eptq_host", str(HOST_PATH))
+        spec = importlib.util.spec_from_file_location("_eptq_host", str(HOST_PATH), loader=loader)
+        mod = importlib.util.module_from_spec(spec)
+        loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def check(status: int, what: str) -> None:

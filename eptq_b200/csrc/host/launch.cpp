@@ -1,0 +1,304 @@
+// Host path of EPTQLinear calls: tensor checks, scratch lookup, output allocation and the C-ABI call in one
+// native function per call.
+//
+// What bounds a small layer's call is this path, not the kernel: written in Python over ctypes it took 23 us per
+// call (module attribute lookups of five buffers, two scratch-size calls, descriptor structures rebuilt for every
+// grouped call) beside kernels of 3 to 10 us.  A LayerHandle keeps the EptqLayer descriptor of a module's device
+// buffers; a call checks by identity that the module still holds those buffers and then only touches the ATen
+// allocator and the library.
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/csrc/Exceptions.h>
+#include <ATen/ATen.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include <map>
+#include <utility>
+#include <vector>
+
+#include "../../../include/eptq_b200.h"
+
+namespace {
+
+constexpr const char* kCapsule = "eptq_b200.LayerHandle";
+constexpr const char* kBufferNames[3] = {"Q", "g", "h"};
+constexpr size_t kMinScratch = 1u << 20;
+constexpr int kSmallRows = 16;
+
+struct LayerHandle {
+    EptqLayer d;
+    PyObject* keep;                     // tensors (and host tables) the descriptor points into
+    PyObject* buffers;                  // the module's _buffers dict
+    PyObject* held[3];                  // Q, g, h as they were when the descriptor was made (owned)
+    const void* held_ptr[3];
+    int64_t in_features, out_features;
+    size_t scratch[kSmallRows + 1];     // eptq_layer_workspace_bytes for small batches, 0 = not asked yet
+};
+
+void free_handle(PyObject* capsule) {
+    auto* h = static_cast<LayerHandle*>(PyCapsule_GetPointer(capsule, kCapsule));
+    if (h == nullptr) { PyErr_Clear(); return; }
+    Py_XDECREF(h->keep);
+    Py_XDECREF(h->buffers);
+    for (PyObject* o : h->held) Py_XDECREF(o);
+    delete h;
+}
+
+LayerHandle* handle_of(PyObject* o) { return static_cast<LayerHandle*>(PyCapsule_GetPointer(o, kCapsule)); }
+
+// The module still holds the buffers the descriptor was made from (replacing or moving one makes a new tensor or
+// a new address).
+bool is_current(const LayerHandle* h) {
+    for (int i = 0; i < 3; ++i) {
+        PyObject* now = PyDict_GetItemString(h->buffers, kBufferNames[i]);        // borrowed
+        if (now != h->held[i] || THPVariable_Unpack(now).const_data_ptr() != h->held_ptr[i]) return false;
+    }
+    return true;
+}
+
+// One zero-filled scratch tensor per (device, stream), grown on demand; only touched with the GIL held.
+std::map<std::pair<int, int64_t>, at::Tensor>& scratch_map() {
+    static auto* m = new std::map<std::pair<int, int64_t>, at::Tensor>();         // never destroyed: no CUDA calls at exit
+    return *m;
+}
+
+const at::Tensor& scratch_for(int device, const c10::cuda::CUDAStream& stream, size_t bytes) {
+    at::Tensor& t = scratch_map()[{device, static_cast<int64_t>(reinterpret_cast<intptr_t>(stream.stream()))}];
+    if (!t.defined() || static_cast<size_t>(t.numel()) < bytes) {
+        const int64_t n = static_cast<int64_t>(bytes > kMinScratch ? bytes : kMinScratch);
+        t = at::zeros({n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+    }
+    return t;
+}
+
+bool fail(int status, const char* what) {
+    PyErr_Format(PyExc_RuntimeError, "%s: %s (eptq status %d)", what, eptq_strerror(status), status);
+    return false;
+}
+
+// x as contiguous fp16 rows of in_features; false with a Python error set if it cannot be.
+bool as_rows(const LayerHandle* h, const at::Tensor& x, at::Tensor& rows, int64_t& n_rows) {
+    if (!x.is_cuda()) {
+        PyErr_SetString(PyExc_RuntimeError, "EPTQLinear runs on CUDA tensors only (there is no CPU path)");
+        return false;
+    }
+    if (x.dim() < 1 || x.size(-1) != h->in_features) {
+        PyErr_Format(PyExc_RuntimeError, "EPTQLinear: the last dimension of the input must be %lld", (long long)h->in_features);
+        return false;
+    }
+    rows = x.scalar_type() == at::kHalf ? x : x.to(at::kHalf);
+    if (!rows.is_contiguous()) rows = rows.contiguous();
+    n_rows = h->in_features > 0 ? rows.numel() / h->in_features : 0;
+    return true;
+}
+
+at::Tensor new_output(const LayerHandle* h, const at::Tensor& x) {
+    at::DimVector shape(x.sizes().begin(), x.sizes().end());
+    shape.back() = h->out_features;
+    return at::empty(shape, x.options().dtype(at::kHalf));
+}
+
+PyObject* wrap(at::Tensor y, at::ScalarType dtype) {
+    return THPVariable_Wrap(dtype == at::kHalf ? std::move(y) : y.to(dtype));
+}
+
+// make_handle(descriptor bytes, keep, buffers dict, in_features, out_features)
+PyObject* make_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    if (n != 5 || !PyBytes_Check(a[0]) || PyBytes_GET_SIZE(a[0]) != static_cast<Py_ssize_t>(sizeof(EptqLayer)) || !PyDict_Check(a[2])) {
+        PyErr_SetString(PyExc_TypeError, "make_handle(descriptor, keep, buffers, in_features, out_features)");
+        return nullptr;
+    }
+    const long long in = PyLong_AsLongLong(a[3]), out = PyLong_AsLongLong(a[4]);
+    if (PyErr_Occurred()) return nullptr;
+    PyObject* held[3];
+    for (int i = 0; i < 3; ++i) {
+        held[i] = PyDict_GetItemString(a[2], kBufferNames[i]);
+        if (held[i] == nullptr || !THPVariable_Check(held[i])) {
+            PyErr_SetString(PyExc_TypeError, "make_handle: buffers Q, g and h must be tensors");
+            return nullptr;
+        }
+    }
+    auto* h = new LayerHandle();
+    std::memcpy(&h->d, PyBytes_AS_STRING(a[0]), sizeof(EptqLayer));
+    h->keep = Py_NewRef(a[1]);
+    h->buffers = Py_NewRef(a[2]);
+    for (int i = 0; i < 3; ++i) {
+        h->held[i] = Py_NewRef(held[i]);
+        h->held_ptr[i] = THPVariable_Unpack(held[i]).const_data_ptr();
+    }
+    h->in_features = in;
+    h->out_features = out;
+    PyObject* c = PyCapsule_New(h, kCapsule, free_handle);
+    if (c == nullptr) delete h;
+    return c;
+}
+
+// forward(handle, x) -> y, or None if the module's buffers are no longer the descriptor's
+PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    LayerHandle* h = n == 2 ? handle_of(a[0]) : nullptr;
+    if (h == nullptr || !THPVariable_Check(a[1])) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "forward(handle, tensor)");
+        return nullptr;
+    }
+    if (!is_current(h)) Py_RETURN_NONE;
+    const at::Tensor& x = THPVariable_Unpack(a[1]);
+    at::Tensor rows;
+    int64_t B = 0;
+    if (!as_rows(h, x, rows, B)) return nullptr;
+    const c10::cuda::OptionalCUDAGuard guard(x.device());
+    at::Tensor y = new_output(h, x);
+    if (B == 0) return wrap(std::move(y), x.scalar_type());
+    const auto stream = c10::cuda::getCurrentCUDAStream(x.device().index());
+    size_t need = B <= kSmallRows ? h->scratch[B] : 0;
+    if (need == 0) {
+        need = eptq_layer_workspace_bytes(&h->d, static_cast<int>(B));
+        if (B <= kSmallRows) h->scratch[B] = need;
+    }
+    const at::Tensor& ws = scratch_for(x.device().index(), stream, need);
+    void* const ws_ptr = ws.data_ptr();
+    const size_t ws_bytes = static_cast<size_t>(ws.numel());
+    const auto* xp = static_cast<const uint16_t*>(rows.const_data_ptr());
+    auto* yp = static_cast<uint16_t*>(y.data_ptr());
+    const EptqLayer d = h->d;
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = eptq_linear_forward(&d, xp, yp, static_cast<int>(B), ws_ptr, ws_bytes, stream.stream());
+    Py_END_ALLOW_THREADS
+    if (st != EPTQ_OK) { fail(st, "eptq linear forward"); return nullptr; }
+    return wrap(std::move(y), x.scalar_type());
+    END_HANDLE_TH_ERRORS
+}
+
+// forward_group(handles, xs) -> list of outputs, or None if some module's buffers have changed.  All inputs have
+// the leading shape of the first.
+PyObject* forward_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
+    HANDLE_TH_ERRORS
+    if (n_args != 2 || !PyList_Check(a[0]) || !PyList_Check(a[1]) || PyList_GET_SIZE(a[0]) != PyList_GET_SIZE(a[1]) ||
+        PyList_GET_SIZE(a[0]) < 1) {
+        PyErr_SetString(PyExc_TypeError, "forward_group(list of handles, list of as many tensors)");
+        return nullptr;
+    }
+    const int n = static_cast<int>(PyList_GET_SIZE(a[0]));
+    std::vector<EptqLayer> descs(n);
+    std::vector<at::Tensor> rows(n), ys(n);
+    std::vector<const uint16_t*> xp(n);
+    std::vector<uint16_t*> yp(n);
+    int64_t B = 0;
+    c10::Device device(c10::kCPU);
+    c10::cuda::OptionalCUDAGuard guard;
+    at::DimVector lead;
+    for (int i = 0; i < n; ++i) {
+        LayerHandle* h = handle_of(PyList_GET_ITEM(a[0], i));
+        PyObject* xo = PyList_GET_ITEM(a[1], i);
+        if (h == nullptr || !THPVariable_Check(xo)) {
+            if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "forward_group: handles and tensors expected");
+            return nullptr;
+        }
+        if (!is_current(h)) Py_RETURN_NONE;
+        const at::Tensor& x = THPVariable_Unpack(xo);
+        int64_t b = 0;
+        if (!as_rows(h, x, rows[i], b)) return nullptr;
+        if (i == 0) {
+            B = b;
+            device = x.device();
+            guard.set_device(device);
+            lead.assign(x.sizes().begin(), x.sizes().end());
+        } else if (b != B || x.device() != device) {
+            PyErr_SetString(PyExc_RuntimeError, "eptq_b200: grouped inputs need one row count and one device");
+            return nullptr;
+        }
+        lead.back() = h->out_features;
+        ys[i] = at::empty(lead, x.options().dtype(at::kHalf));
+        descs[i] = h->d;
+        xp[i] = static_cast<const uint16_t*>(rows[i].const_data_ptr());
+        yp[i] = static_cast<uint16_t*>(ys[i].data_ptr());
+    }
+    const size_t need = eptq_group_workspace_bytes(descs.data(), n, static_cast<int>(B));
+    if (need == 0) {
+        PyErr_SetString(PyExc_RuntimeError, "eptq_b200: this set of layers cannot run as one group launch");
+        return nullptr;
+    }
+    const auto stream = c10::cuda::getCurrentCUDAStream(device.index());
+    const at::Tensor& ws = scratch_for(device.index(), stream, need);
+    void* const ws_ptr = ws.data_ptr();
+    const size_t ws_bytes = static_cast<size_t>(ws.numel());
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = eptq_linear_forward_group(descs.data(), n, xp.data(), yp.data(), static_cast<int>(B), ws_ptr, ws_bytes, stream.stream());
+    Py_END_ALLOW_THREADS
+    if (st != EPTQ_OK) { fail(st, "eptq group forward"); return nullptr; }
+    PyObject* out = PyList_New(n);
+    if (out == nullptr) return nullptr;
+    for (int i = 0; i < n; ++i)
+        PyList_SET_ITEM(out, i, wrap(std::move(ys[i]), THPVariable_Unpack(PyList_GET_ITEM(a[1], i)).scalar_type()));
+    return out;
+    END_HANDLE_TH_ERRORS
+}
+
+// dequantize(handle) -> fp16 (out, in) weight, or None if the module's buffers have changed
+PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    LayerHandle* h = n == 1 ? handle_of(a[0]) : nullptr;
+    if (h == nullptr) {
+        if (!PyErr_Occurred()) PyErr_SetString(PyExc_TypeError, "dequantize(handle)");
+        return nullptr;
+    }
+    if (!is_current(h)) Py_RETURN_NONE;
+    const at::Tensor& q = THPVariable_Unpack(h->held[0]);
+    if (!q.is_cuda()) {
+        PyErr_SetString(PyExc_RuntimeError, "eptq_b200: `Q` must be a CUDA tensor (no CPU path exists)");
+        return nullptr;
+    }
+    const c10::cuda::OptionalCUDAGuard guard(q.device());
+    at::Tensor w = at::empty({h->out_features, h->in_features}, q.options().dtype(at::kHalf));
+    const auto stream = c10::cuda::getCurrentCUDAStream(q.device().index());
+    auto* wp = static_cast<uint16_t*>(w.data_ptr());
+    const EptqLayer d = h->d;
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = eptq_dequantize(&d, wp, stream.stream());
+    Py_END_ALLOW_THREADS
+    if (st != EPTQ_OK) { fail(st, "eptq dequantize"); return nullptr; }
+    return THPVariable_Wrap(std::move(w));
+    END_HANDLE_TH_ERRORS
+}
+
+// scratch(device index, bytes) -> the scratch tensor of the current stream
+PyObject* scratch(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 2) { PyErr_SetString(PyExc_TypeError, "scratch(device index, bytes)"); return nullptr; }
+    const long device = PyLong_AsLong(a[0]);
+    const size_t bytes = PyLong_AsSize_t(a[1]);
+    if (PyErr_Occurred()) return nullptr;
+    const c10::cuda::OptionalCUDAGuard guard(c10::Device(c10::kCUDA, static_cast<c10::DeviceIndex>(device)));
+    return THPVariable_Wrap(scratch_for(static_cast<int>(device), c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(device)), bytes));
+    END_HANDLE_TH_ERRORS
+}
+
+// scratch_of_device(device index) -> list of all its scratch tensors (one per stream that ran the kernels)
+PyObject* scratch_of_device(PyObject*, PyObject* const* a, Py_ssize_t n) {
+    HANDLE_TH_ERRORS
+    if (n != 1) { PyErr_SetString(PyExc_TypeError, "scratch_of_device(device index)"); return nullptr; }
+    const long device = PyLong_AsLong(a[0]);
+    if (PyErr_Occurred()) return nullptr;
+    PyObject* out = PyList_New(0);
+    if (out == nullptr) return nullptr;
+    for (auto& kv : scratch_map()) {
+        if (kv.first.first != device) continue;
+        PyObject* t = THPVariable_Wrap(kv.second);
+        if (t == nullptr || PyList_Append(out, t) != 0) { Py_XDECREF(t); Py_DECREF(out); return nullptr; }
+        Py_DECREF(t);
+    }
+    return out;
+    END_HANDLE_TH_ERRORS
+}
+
+#define METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(name)), METH_FASTCALL, nullptr}
+PyMethodDef methods[] = {METHOD(make_handle), METHOD(forward), METHOD(forward_group), METHOD(dequantize),
+                         METHOD(scratch), METHOD(scratch_of_device), {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_eptq_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__eptq_host(void) { return PyModule_Create(&module); }

@@ -25,21 +25,14 @@ from .. import _lib
 __all__ = ["e8_forward", "e8d4_forward", "linear_forward", "linear_forward_group", "linear_forward_chain",
            "dequantize_layer", "workspace_for", "workspace_status", "workspace_status_all"]
 
-_workspaces: Dict[Tuple[int, int], torch.Tensor] = {}
-
 
 def workspace_for(device: torch.device, nbytes: int) -> torch.Tensor:
     """Zero-initialised scratch for (device, current stream), grown on demand.
 
     Calls ordered on one stream share it; the kernels leave it zeroed where they
     need zeros.  Growing allocates, so size it before capturing a CUDA graph."""
-    stream = torch.cuda.current_stream(device)
-    key = (device.index if device.index is not None else torch.cuda.current_device(), stream.cuda_stream)
-    ws = _workspaces.get(key)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.zeros(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-        _workspaces[key] = ws
-    return ws
+    index = device.index if device.index is not None else torch.cuda.current_device()
+    return _lib.host().scratch(index, nbytes)
 
 
 def _require_cuda(**tensors) -> None:
@@ -407,10 +400,9 @@ def workspace_status_all(device) -> int:
     dev = torch.device(device)
     index = dev.index if dev.index is not None else torch.cuda.current_device()
     first = 0
-    for (d, _stream_id), ws in list(_workspaces.items()):
-        if d == index:
-            code = workspace_status(ws)
-            first = first or code
+    for ws in _lib.host().scratch_of_device(index):
+        code = workspace_status(ws)
+        first = first or code
     return first
 
 

@@ -21,10 +21,8 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-import ctypes as C
-
 from .. import _lib
-from . import _make_desc, critical_lists, d4_table8, dequantize_layer, linear_forward, linear_forward_group, workspace_for
+from . import _make_desc, critical_lists, d4_table8, linear_forward
 
 MARKER = 32767     # int16 value that marks a critical block (index 65535 - 32768)
 
@@ -100,11 +98,11 @@ class EPTQLinear(nn.Module):
         # Shared between layers, therefore plain attributes, not buffers.
         self._codebook = codebook
         self._codebook32 = codebook32
-        self._desc = None            # cached C-ABI descriptor, dropped whenever the buffers may have moved
+        self._handle = None          # descriptor of the device buffers for the native host path
 
     def _apply(self, fn, *args, **kwargs):
         super()._apply(fn, *args, **kwargs)
-        self._desc = None
+        self._handle = None
         self._codebook = self._move_shared(self._codebook, fn)
         if self._codebook32 is not None:
             moved = self._move_shared(self._codebook32, fn)
@@ -155,6 +153,13 @@ class EPTQLinear(nn.Module):
         )
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
+        if torch.compiler.is_compiling():
+            return self._forward_traced(x)
+        y = None if self._handle is None else _lib.host().forward(self._handle, x)
+        return y if y is not None else _lib.host().forward(self._new_handle(), x)
+
+    def _forward_traced(self, x: torch.Tensor) -> torch.Tensor:
+        """Under torch.compile: through the registered custom op (one graph node, has a fake implementation)."""
         if not x.is_cuda:
             raise RuntimeError("EPTQLinear runs on CUDA tensors only (there is no CPU path)")
         lead, out_dtype = x.shape[:-1], x.dtype
@@ -163,46 +168,34 @@ class EPTQLinear(nn.Module):
             x2 = x2.half()
         if not x2.is_contiguous():
             x2 = x2.contiguous()
-        if torch.compiler.is_compiling():
-            # traced: go through the registered custom op (one graph node, has a fake implementation)
-            y = linear_forward(x2, self.Q, self._codebook, self._codebook32, self.g, self.h,
-                               self.O_vals, self.O_col, self.O_row_ptr, self.bias, self.S_group,
-                               self.quantizer_type, self.qb_size)
-        else:
-            y = self._forward_direct(x2)
+        y = linear_forward(x2, self.Q, self._codebook, self._codebook32, self.g, self.h,
+                           self.O_vals, self.O_col, self.O_row_ptr, self.bias, self.S_group,
+                           self.quantizer_type, self.qb_size)
         if out_dtype != torch.float16:
             y = y.to(out_dtype)
         return y.reshape(*lead, self.out_features)
 
-    def _forward_direct(self, x2: torch.Tensor) -> torch.Tensor:
-        """Eager path: cached descriptor, one ctypes call, no dispatcher in between."""
-        lib = _lib.load()
-        d = self._desc
-        if d is None or d.Q != self.Q.data_ptr() or d.h != self.h.data_ptr() or d.g != self.g.data_ptr():
-            d = self._desc = self.descriptor()
-        B = x2.shape[0]
-        y = torch.empty((B, self.out_features), dtype=torch.float16, device=x2.device)
-        if B == 0:
-            return y
-        ws = workspace_for(x2.device, lib.eptq_layer_workspace_bytes(C.byref(d), B))
-        if x2.device.index is not None and x2.device.index != torch.cuda.current_device():
-            with torch.cuda.device(x2.device):
-                st = lib.eptq_linear_forward(C.byref(self._desc), x2.data_ptr(), y.data_ptr(), B, ws.data_ptr(),
-                                             ws.numel(), torch.cuda.current_stream(x2.device).cuda_stream)
-        else:
-            st = lib.eptq_linear_forward(C.byref(self._desc), x2.data_ptr(), y.data_ptr(), B, ws.data_ptr(),
-                                         ws.numel(), torch.cuda.current_stream(x2.device).cuda_stream)
-        if st != 0:
-            _lib.check(st, "eptq linear forward")
-        return y
+    def _new_handle(self):
+        """Native handle of the current buffers; the host path says (by returning None) when they have been
+        replaced or moved since, and a new one is made."""
+        if not self.Q.is_cuda:
+            raise RuntimeError("EPTQLinear runs on CUDA tensors only (there is no CPU path)")
+        d = self.descriptor()
+        keep = (d, tuple(self._buffers.values()), self._codebook, self._codebook32)
+        self._handle = _lib.host().make_handle(bytes(d), keep, self._buffers, self.in_features, self.out_features)
+        return self._handle
+
+    def __getstate__(self):
+        state = super().__getstate__() if hasattr(super(), "__getstate__") else self.__dict__
+        return {**state, "_handle": None}          # a copy describes its own buffers
 
     def dequantize(self) -> torch.Tensor:
         """fp16 (out, in) weight reconstructed on the GPU, bit-identical to the
         reference's ``dequantize_layer`` when the layer was built from an fp32 codebook."""
         if self._codebook32 is None:
             raise RuntimeError("this layer was built from an fp16 codebook; exact reconstruction needs the fp32 table")
-        return dequantize_layer(self.Q, self._codebook32, self.g, self.h, self.O_vals, self.O_col,
-                                self.O_row_ptr, self.S_group, self.quantizer_type, self.qb_size)
+        w = None if self._handle is None else _lib.host().dequantize(self._handle)
+        return w if w is not None else _lib.host().dequantize(self._new_handle())
 
     def descriptor(self):
         """The C-ABI description (struct EptqLayer) of this layer's device buffers."""
@@ -219,16 +212,10 @@ def forward_group(layers, xs):
     """Apply several independent EPTQLinear layers in one kernel launch: layers[i](xs[i]) for all i.
     Inputs need one common leading shape with at most 16 rows; the layers must share one codebook and have no
     group scales.  Returns the list of outputs.  Meant for q/k/v and gate/up."""
-    lead = xs[0].shape[:-1]
-    x2 = []
-    for lin, x in zip(layers, xs):
-        if not x.is_cuda:
-            raise RuntimeError("EPTQLinear runs on CUDA tensors only (there is no CPU path)")
-        v = x.reshape(-1, lin.in_features)
-        v = v if v.dtype == torch.float16 else v.half()
-        x2.append(v if v.is_contiguous() else v.contiguous())
-    ys = linear_forward_group([lin.descriptor() for lin in layers], x2, [lin.out_features for lin in layers])
-    return [y.to(x.dtype).reshape(*lead, lin.out_features) for y, x, lin in zip(ys, xs, layers)]
+    host = _lib.host()
+    handles = [lin._handle or lin._new_handle() for lin in layers]
+    ys = host.forward_group(handles, list(xs))
+    return ys if ys is not None else host.forward_group([lin._new_handle() for lin in layers], list(xs))
 
 
 QuantizedLinear = EPTQLinear
