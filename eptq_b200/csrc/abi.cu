@@ -101,8 +101,8 @@ int forward_checked(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B,
     if (big_enough && group_gemv_supported(&L, 1, B) && aligned16(y)) {
         const uint16_t* xs[1] = {x};
         uint16_t* ys[1] = {y};
-        const size_t need = group_workspace_bytes(&L, 1, B, 0);
-        if (need != 0 && workspace != nullptr && workspace_bytes >= need)
+        // The least it runs with; above two rows more scratch means fewer passes (launch_gemv_group).
+        if (group_workspace_bytes(&L, 1, B, 0) != 0 && workspace != nullptr && workspace_bytes >= kPartialOffset)
             return launch_gemv_group(&L, 1, nullptr, xs, ys, B, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
     }
     if (mma_gemv_supported(L, B) && aligned16(L.g) && (L.bias == nullptr || aligned16(L.bias)) && aligned16(y))

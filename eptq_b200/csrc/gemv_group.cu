@@ -48,6 +48,10 @@
 
 namespace eptq {
 
+size_t rows_workspace_bytes(const EptqLayer* layers, int n, int B, int n_sms);
+int launch_gemv_rows(const EptqLayer* layers, int n, const uint16_t* const* xs, uint16_t* const* ys, int B, int n_sms,
+                     void* workspace, cudaStream_t stream);
+
 using namespace groupdev;
 
 
@@ -603,7 +607,7 @@ bool group_layer_supported(const EptqLayer& L) {
 }  // namespace
 
 bool group_gemv_supported(const EptqLayer* layers, int n, int B) {
-    if (layers == nullptr || n < 1 || n > kMaxGroupLayers || B < 1 || B > kGemmMinBatch) return false;   // > 2: passes of two rows
+    if (layers == nullptr || n < 1 || n > kMaxGroupLayers || B < 1 || B > kGemmMinBatch) return false;
     for (int i = 0; i < n; ++i) {
         if (!group_layer_supported(layers[i])) return false;
         if (layers[i].quantizer != layers[0].quantizer || layers[i].table16 != layers[0].table16 ||
@@ -617,7 +621,8 @@ size_t group_workspace_bytes(const EptqLayer* layers, int n, int B, int n_sms) {
     GroupPlan plan;
     if (n_sms <= 0) n_sms = 148;
     if (!plan_group(layers, n, B > 2 ? 2 : B, n_sms, plan)) return 0;
-    return kPartialOffset;
+    const size_t rows = B > 2 ? rows_workspace_bytes(layers, n, B, n_sms) : 0;      // what one pass for all rows wants
+    return rows > kPartialOffset ? rows : kPartialOffset;
 }
 
 namespace {
@@ -673,13 +678,18 @@ int launch_gemv_group_pass(const EptqLayer* layers, int n, const EptqFusion* fus
 
 }  // namespace
 
-// Batches above 2 run as passes of two batch rows over the same weights (the kernel's MMA columns hold two
-// rows); the scratch is reused, the passes are ordered on the stream.  Fused epilogues that index a cache
-// by batch entry are limited to one pass.
+// Batches above 2 take one pass for all rows (gemv_rows.cu) when the scratch has room for its partial sums; otherwise
+// passes of two batch rows over the same weights (this kernel's MMA columns hold two rows), the scratch reused, the
+// passes ordered on the stream.  Two rows stay here: one launch either way, 31.3 against 37.1 us for gate/up of a 7B
+// model in E8-D4, 42.8 against 60.8 us in E8.  Fused epilogues that index a cache by batch entry are limited to one pass.
 int launch_gemv_group(const EptqLayer* layers, int n, const EptqFusion* fusions, const uint16_t* const* xs,
                       uint16_t* const* ys, int B, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
     if (B <= 2) return launch_gemv_group_pass(layers, n, fusions, xs, ys, B, workspace, workspace_bytes, stream);
     if (fusions != nullptr || n > kMaxGroupLayers) return EPTQ_ERR_UNSUPPORTED;
+    const int n_sms = cached_sm_count();
+    const size_t rows = rows_workspace_bytes(layers, n, B, n_sms);
+    if (rows != 0 && workspace != nullptr && workspace_bytes >= rows)
+        return launch_gemv_rows(layers, n, xs, ys, B, n_sms, workspace, stream);
     const uint16_t* xp[kMaxGroupLayers];
     uint16_t* yp[kMaxGroupLayers];
     for (int b0 = 0; b0 < B; b0 += 2) {

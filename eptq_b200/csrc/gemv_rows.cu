@@ -1,0 +1,670 @@
+// Decode GEMV of 3 to 16 batch rows over a group of independent layers of one codebook (E8-D4 or E8), one pass
+// over the weights.
+//
+// What bounds it: decoding an index (two conflict-free table reads of 2 wavefronts each for E8-D4, one conflicting
+// read for E8, about eight integer instructions) costs more than streaming its two bytes, so every decoded
+// codeword has to serve all batch rows.  The two-row kernel of gemv_group.cu, run once per pair of rows, decoded
+// every index ceil(B / 2) times and left seven eighths of each MMA's columns to a diagonal.  Here a pair of
+// codewords of neighbouring columns is transposed with PRMT (4 instructions per index) into ordinary A fragments
+// (16 outputs x 16 columns), and the MMA columns are batch rows.
+//
+// Arithmetic as in gemv_group.cu: codewords unmodified in fp16, x*h*2^-e split into an fp16 part and an fp16
+// remainder, fp32 accumulation.  NB = 4: the remainders take columns 4..7 of the one column tile; NB = 8, 16: they
+// run as a second MMA into the same accumulators.
+//
+// Work split: a step is 32 Q rows x 32 columns; all steps (layer, row tile, column step) form one sequence, block b
+// takes the contiguous share [W*b/G, W*(b+1)/G).  16 main warps: warp = (column group kq = warp / 4, row group
+// rg = warp % 4); the four warps of a column group take every fourth step of the share, convert the step's
+// activations once into a shared fragment buffer (double-buffered, one 128-thread barrier per step) and each decode 8
+// Q rows.  At the end of a row tile (or of the share) the four column groups are added through shared memory and
+// the block's partial sums go to scratch with plain stores; the block (or, for a unit of corrections, warp) that takes the last
+// ticket of a row tile adds the partials in block order, so results do not depend on arrival order.
+//
+// Critical blocks: while the table arrives, the warps of the launch walk the CSR tables in units of 4 Q rows (at most a
+// unit or two per warp for the fractions in use) and store sum (O - code[65535])*h*x to a slot of their own that the
+// last arrival adds.  Dedicated warps for it would leave 96 registers a thread, and the main loop then spills: to L2,
+// since nearly all of L1 is shared memory (4096 x 4096 E8-D4, 16 rows: 60.3 against 23.7 us a call).
+
+#include <atomic>
+#include <cmath>
+#include <mutex>
+
+#include "common.cuh"
+
+namespace eptq {
+
+namespace {
+
+constexpr int kRowsMaxLayers = 32;
+constexpr int kRowsFewLayers = 8;          // launches of few layers copy a smaller parameter block
+constexpr int kTileRows = 32;              // Q rows of a row tile (256 outputs)
+constexpr int kTileOut = kTileRows * 8;
+constexpr int kColGroups = 4;
+constexpr int kRowsWarps = 16;
+constexpr int kRowsThreads = kRowsWarps * 32;
+// Steps of Q, x and h in flight per warp.  Two cover the memory latency where a step is long (16 rows), and the
+// registers of a third would spill there.
+__host__ __device__ constexpr int ring_steps(int nb) { return nb == 16 ? 2 : 3; }
+constexpr int kCorrPerTile = kTileRows / 4;
+constexpr unsigned kRowsTableAddr = 0x10000u;                   // shared-window address of the replicated E8-D4 table
+constexpr int kRowsSmemD4 = 2 * 65536 - 1024;                   // window [0x400, 0x20000)
+constexpr int kRowsSmemE8 = 232448;                             // the most a block may ask for
+constexpr unsigned kCtrlBytes = 64;
+
+// Fragment buffers ([column group][2][hi, lo][NB rows][32 columns] fp16), reused for the sum over column groups.
+__host__ __device__ constexpr unsigned area_bytes(int nb) { return nb == 16 ? 16384u : 8192u; }
+__host__ __device__ constexpr unsigned e8_table_offset(int nb) { return area_bytes(nb) + kCtrlBytes; }
+__host__ __device__ constexpr unsigned e8_resident(int nb) { return (kRowsSmemE8 - e8_table_offset(nb)) / 4; }
+
+struct RowsLayer {
+    const int16_t* Q;
+    const __half* g;
+    const __half* h;
+    const __half* x;
+    const __half* O_vals;
+    const int* O_col;
+    const int* O_row_ptr;
+    const __half* bias;
+    __half* y;
+    int step0;              // index of this layer's first step
+    int tile0;              // index of its first row tile
+    int corr0;              // index of its first correction unit
+    int M, N;
+    int ns;                 // steps per row tile = N / 32
+    int row_tiles;          // ceil(M / 32)
+    int corr_tile;          // correction units per row tile: 8, or 0 for a layer without critical blocks
+    float x_scale;          // power of two, <= 1 / max|h|
+    float x_inv_scale;
+};
+
+template <int MAXL>
+struct RowsArgs {
+    RowsLayer L[MAXL];
+    const uint2* table16;
+    const unsigned* packed;
+    unsigned* counters;     // zero on entry, zero again on exit
+    float* partial;         // [block + tile][NB][256] main partials, then [tile][NB][256] corrections
+    unsigned W;             // steps
+    int G;                  // blocks with a share
+    int tiles;
+    int corr_units;
+    int n_layers;
+    int B;
+};
+
+__device__ __forceinline__ uint2 lds64(unsigned addr) {
+    uint2 v;
+    asm volatile("ld.shared.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr));
+    return v;
+}
+__device__ __forceinline__ unsigned lo_halves(unsigned a, unsigned b) { return __byte_perm(a, b, 0x5410); }
+__device__ __forceinline__ unsigned hi_halves(unsigned a, unsigned b) { return __byte_perm(a, b, 0x7632); }
+__device__ __forceinline__ void mma(float (&c)[4], const unsigned (&a)[4], unsigned b0, unsigned b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+                 : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ uint4 ldg_once(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void split_half(float v, __half& hi, __half& lo) {
+    hi = __float2half_rn(v);
+    lo = __float2half_rn(v - __half2float(hi));
+}
+
+// Packed E8 entry -> fp16 pairs of dims (0,1), (2,3), (4,5), (6,7): the layout and the arithmetic are stated at
+// e8_decode in gemv_group.cu.
+__device__ __forceinline__ void e8_entry(unsigned e, unsigned (&r)[4]) {
+    const unsigned rot = __funnelshift_r(e, e, 8);
+    const unsigned magic = 0x64006400u;
+    unsigned a[4] = {(e & 0x003C003Cu) | magic, (e & 0x03C003C0u) | magic, (rot & 0x003C003Cu) | magic, (rot & 0x03C003C0u) | magic};
+    const __half2 kA = __floats2half2_rn(0.125f, 0.125f), cA = __floats2half2_rn(-131.f, -131.f);
+    const __half2 kB = __floats2half2_rn(0.0078125f, 0.0078125f), cB = __floats2half2_rn(-11.f, -11.f);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const __half2 v = __hfma2(*reinterpret_cast<__half2*>(&a[i]), i & 1 ? kB : kA, i & 1 ? cB : cA);
+        r[i] = *reinterpret_cast<const unsigned*>(&v);
+    }
+}
+template <int NB>
+__device__ __forceinline__ unsigned e8_fetch(unsigned u, unsigned tbase, const unsigned* packed) {
+    unsigned v;
+    asm volatile("{\n\t.reg .pred p;\n\t.reg .u64 ga;\n\t.reg .u32 sa;\n\t"
+                 "setp.ge.u32 p, %1, %2;\n\t"
+                 "mad.wide.u32 ga, %1, 4, %3;\n\t"
+                 "mad.lo.u32 sa, %1, 4, %4;\n\t"
+                 "@p ld.global.nc.u32 %0, [ga];\n\t"
+                 "@!p ld.shared.u32 %0, [sa];\n\t}"
+                 : "=r"(v) : "r"(u), "n"(e8_resident(NB)), "l"(packed), "r"(tbase));
+    return v;
+}
+
+// Block that owns step s when block b owns [b*W/G, (b+1)*W/G); the host keeps W * G below 2^32.
+__device__ __forceinline__ int owner_block(unsigned s, unsigned W, unsigned G) {
+    unsigned b = (s * G) / W;
+    while (b + 1 < G && ((b + 1) * W) / G <= s) ++b;
+    while (b > 0 && (b * W) / G > s) --b;
+    return static_cast<int>(b);
+}
+
+// Adds the partial sums of a row tile in block order, then the corrections; writes y.  Run by `n` threads.
+template <int NB, int MAXL>
+__device__ __forceinline__ void finish_tile(const RowsArgs<MAXL>& p, const RowsLayer& L, int rt, int tid, int n) {
+    const int tile = L.tile0 + rt;
+    if (tid == 0) p.counters[tile] = 0u;
+    const unsigned s0 = static_cast<unsigned>(L.step0 + rt * L.ns);
+    const int first = owner_block(s0, p.W, p.G), last = owner_block(s0 + L.ns - 1, p.W, p.G);
+    const size_t slot = static_cast<size_t>(NB) * kTileOut;
+    const float* parts = p.partial + (first + tile) * slot;
+    const float* corr = L.corr_tile != 0 ? p.partial + (p.G + p.tiles + tile) * slot : nullptr;
+    for (int i = tid; i < p.B * (kTileOut / 4); i += n) {
+        const int b = i / (kTileOut / 4), q = i % (kTileOut / 4);
+        if (rt * kTileRows + (q >> 1) >= L.M) continue;
+        const size_t off = static_cast<size_t>(b) * kTileOut + q * 4;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        int k = 0;
+        for (; k + 4 <= last - first + 1; k += 4) {                     // four loads in flight
+            float4 v[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = __ldcg(reinterpret_cast<const float4*>(parts + (k + j) * slot + off));
+#pragma unroll
+            for (int j = 0; j < 4; ++j) { s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w; }
+        }
+        for (; k <= last - first; ++k) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(parts + k * slot + off));
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        if (corr != nullptr) {
+            const float4 v = __ldcg(reinterpret_cast<const float4*>(corr + off));
+            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        const int o = rt * kTileOut + q * 4;
+        const uint2 graw = __ldg(reinterpret_cast<const uint2*>(L.g + o));
+        const float2 g01 = __half22float2(*reinterpret_cast<const __half2*>(&graw.x));
+        const float2 g23 = __half22float2(*reinterpret_cast<const __half2*>(&graw.y));
+        float2 b01 = make_float2(0.f, 0.f), b23 = make_float2(0.f, 0.f);
+        if (L.bias != nullptr) {
+            const uint2 braw = __ldg(reinterpret_cast<const uint2*>(L.bias + o));
+            b01 = __half22float2(*reinterpret_cast<const __half2*>(&braw.x));
+            b23 = __half22float2(*reinterpret_cast<const __half2*>(&braw.y));
+        }
+        const __half2 o01 = __floats2half2_rn(fmaf(s.x, g01.x, b01.x), fmaf(s.y, g01.y, b01.y));
+        const __half2 o23 = __floats2half2_rn(fmaf(s.z, g23.x, b23.x), fmaf(s.w, g23.y, b23.y));
+        uint2 ov;
+        ov.x = *reinterpret_cast<const unsigned*>(&o01);
+        ov.y = *reinterpret_cast<const unsigned*>(&o23);
+        *reinterpret_cast<uint2*>(L.y + static_cast<size_t>(b) * 8 * L.M + o) = ov;
+    }
+}
+
+template <int MAXL>
+__device__ __forceinline__ bool last_arrival(const RowsArgs<MAXL>& p, const RowsLayer& L, int rt) {
+    unsigned ticket;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(ticket) : "l"(p.counters + L.tile0 + rt) : "memory");
+    const unsigned s0 = static_cast<unsigned>(L.step0 + rt * L.ns);
+    const int n = owner_block(s0 + L.ns - 1, p.W, p.G) - owner_block(s0, p.W, p.G) + 1;
+    return ticket == static_cast<unsigned>(n + L.corr_tile) - 1u;
+}
+
+// Correction units cw, cw + n_warps, ...: 4 Q rows each, 8 lanes per row, four batch rows at a time.
+template <int KIND, int NB, int MAXL>
+__device__ void run_corrections(const RowsArgs<MAXL>& p, int cw, int n_warps, int lane) {
+    float cstar[4] = {0.f, 0.f, 0.f, 0.f};                     // what the main loop adds for a marker (E8: zero)
+    if (KIND == EPTQ_E8D4) {
+        const uint2 raw = __ldg(p.table16 + 511);
+        const float2 c01 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
+        const float2 c23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
+        cstar[0] = c01.x; cstar[1] = c01.y; cstar[2] = c23.x; cstar[3] = c23.y;
+    }
+    int l = 0;
+    for (int u = cw; u < p.corr_units; u += n_warps) {
+        while (l + 1 < p.n_layers && p.L[l + 1].corr0 <= u) ++l;     // layers without units share their successor's corr0
+        const RowsLayer& L = p.L[l];
+        const int qt = u - L.corr0, rt = qt / kCorrPerTile;
+        const int row = qt * 4 + (lane >> 3), sub = lane & 7;
+        int lo = 0, hi = 0;
+        if (row < L.M) { lo = __ldg(L.O_row_ptr + row); hi = __ldg(L.O_row_ptr + row + 1); }
+        float* dst = p.partial + (static_cast<size_t>(p.G + p.tiles + L.tile0 + rt) * NB) * kTileOut + ((qt % kCorrPerTile) * 4 + (lane >> 3)) * 8;
+        for (int b0 = 0; b0 < p.B; b0 += 4) {
+            float acc[4][8];
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc[b][k] = 0.f;
+            for (int i = lo + sub; i < hi; i += 8) {
+                const int col = __ldg(L.O_col + i);
+                const float hv = __half2float(__ldg(L.h + col));
+                float o8[8];
+                unpack8(ldg128(L.O_vals + static_cast<size_t>(i) * 8), o8);
+                float xv[4];
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+                    xv[b] = b0 + b < p.B ? hv * __half2float(__ldg(L.x + static_cast<size_t>(b0 + b) * L.N + col)) : 0.f;
+#pragma unroll
+                for (int b = 0; b < 4; ++b)
+#pragma unroll
+                    for (int k = 0; k < 8; ++k) acc[b][k] = fmaf(o8[k] - cstar[k & 3], xv[b], acc[b][k]);
+            }
+            __syncwarp();
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) {
+                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 1);
+                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 2);
+                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 4);
+                }
+                if (sub == 0 && b0 + b < p.B) {
+                    float4* d4 = reinterpret_cast<float4*>(dst + static_cast<size_t>(b0 + b) * kTileOut);
+                    __stcg(d4, make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]));
+                    __stcg(d4 + 1, make_float4(acc[b][4], acc[b][5], acc[b][6], acc[b][7]));
+                }
+            }
+        }
+        __syncwarp();
+        int mine = 0;
+        if (lane == 0) mine = last_arrival(p, L, rt);
+        if (__shfl_sync(0xffffffffu, mine, 0)) finish_tile<NB>(p, L, rt, lane, 32);
+        __syncwarp();
+    }
+}
+
+template <int KIND, int NB, int MAXL>
+__global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid_constant__ RowsArgs<MAXL> p) {
+    constexpr int RING = ring_steps(NB);
+    constexpr int BT = NB == 16 ? 2 : 1;                       // accumulator column tiles
+    // Fragment buffer: [16-column half ks][fp16 part, remainder][row][columns 8t + 4ks .. +3 for t = 0..3] fp16, so
+    // that a warp's 64-bit reads of one half are contiguous.
+    constexpr unsigned kLoPlane = NB * 32;                     // bytes from a row's fp16 parts to its remainders
+    constexpr unsigned kHalf = NB * 64;                        // bytes between the halves
+    constexpr unsigned kBuf = NB * 128;                        // one fragment buffer of a column group
+    extern __shared__ __align__(1024) unsigned char smem_raw[];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(smem_raw));     // 0x400: the first KB is reserved
+    if (base != 0x400u) {                                      // the table address is part of the lookup arithmetic
+        if (tid == 0) atomicExch(reinterpret_cast<int*>(p.counters) + (kMaxCounters - 1), static_cast<int>(EPTQ_ERR_LAUNCH));
+        return;
+    }
+    asm volatile("griddepcontrol.launch_dependents;");
+
+    const int g = lane >> 2, t = lane & 3;
+    const int kq = warp >> 2, rg = warp & 3, ctid = tid & 127;
+    const unsigned s_begin = (static_cast<unsigned>(blockIdx.x) * p.W) / p.G;
+    const unsigned s_end = ((static_cast<unsigned>(blockIdx.x) + 1u) * p.W) / p.G;
+
+    // A column group's position: row tile `rt` of layer `l`, its next step k, the end of the block's share of the
+    // tile.  Past the last step l = n_layers.
+    struct Pos { int l, rt; unsigned tile_s0; int k, kend; };
+    auto settle = [&](Pos& c) {                                // move on to the tile that has the group's next step
+        while (c.l < p.n_layers && c.k >= c.kend) {
+            c.tile_s0 += p.L[c.l].ns;
+            if (++c.rt == p.L[c.l].row_tiles) { c.rt = 0; ++c.l; }
+            if (c.tile_s0 >= s_end) { c.l = p.n_layers; return; }
+            c.kend = min(p.L[c.l].ns, static_cast<int>(s_end - c.tile_s0));
+            c.k = kq;
+        }
+    };
+    Pos cur;
+    {
+        int l = 0;
+        while (l + 1 < p.n_layers && static_cast<unsigned>(p.L[l + 1].step0) <= s_begin) ++l;
+        const unsigned local = s_begin - p.L[l].step0, ns = p.L[l].ns;
+        cur.l = l;
+        cur.rt = static_cast<int>(local / ns);
+        cur.tile_s0 = p.L[l].step0 + cur.rt * ns;
+        cur.k = static_cast<int>(s_begin - cur.tile_s0) + kq;
+        cur.kend = min(static_cast<int>(ns), static_cast<int>(s_end - cur.tile_s0));
+    }
+    Pos pf = cur;
+    settle(pf);
+    // prefetch pointers of the position: Q row of this lane, x and h columns this thread converts
+    constexpr int XC = NB == 16 ? 4 : NB == 8 ? 2 : 1;         // columns converted per thread
+    const int xrow = ctid / (32 / XC), xcol = (ctid % (32 / XC)) * XC;
+    const bool xlive = xrow < p.B;
+    struct Raw { uint4 q; unsigned x[(XC + 1) / 2], h[(XC + 1) / 2]; };
+    const int16_t* qp = nullptr;
+    const __half *xp = nullptr, *hp = nullptr;
+    auto place = [&]() {
+        if (pf.l >= p.n_layers) return;
+        const RowsLayer& L = p.L[pf.l];
+        const int row = min(pf.rt * kTileRows + rg * 8 + g, L.M - 1);
+        qp = L.Q + static_cast<size_t>(row) * L.N + pf.k * 32 + 8 * t;
+        xp = L.x + static_cast<size_t>(xlive ? xrow : 0) * L.N + pf.k * 32 + xcol;
+        hp = L.h + pf.k * 32 + xcol;
+    };
+    auto next = [&]() {
+        pf.k += kColGroups;
+        if (pf.k < pf.kend) { qp += 32 * kColGroups; xp += 32 * kColGroups; hp += 32 * kColGroups; }
+        else { settle(pf); place(); }
+    };
+    auto load_cols = [&](const __half* src, unsigned (&v)[(XC + 1) / 2]) {
+        if constexpr (XC == 4) { const uint2 w = __ldg(reinterpret_cast<const uint2*>(src)); v[0] = w.x; v[1] = w.y; }
+        else if constexpr (XC == 2) v[0] = __ldg(reinterpret_cast<const unsigned*>(src));
+        else v[0] = __half_as_ushort(__ldg(src));
+    };
+    Raw ring[RING];
+    place();
+    Pos pf0 = pf;
+#pragma unroll
+    for (int i = 0; i < RING; ++i) {                      // weights do not depend on the previous kernel
+        ring[i].q = make_uint4(0, 0, 0, 0);
+#pragma unroll
+        for (int e = 0; e < (XC + 1) / 2; ++e) { ring[i].x[e] = 0u; ring[i].h[e] = 0u; }
+        if (pf.l < p.n_layers) { ring[i].q = ldg_once(qp); load_cols(hp, ring[i].h); next(); }
+    }
+
+    if constexpr (KIND == EPTQ_E8) {
+        const unsigned dst0 = base + e8_table_offset(NB);
+        const char* src0 = reinterpret_cast<const char*>(p.packed);
+        for (unsigned off = tid * 16u; off < e8_resident(NB) * 4u; off += kRowsThreads * 16u)
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst0 + off), "l"(src0 + off) : "memory");
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    } else {
+        // entry order follows the raw stored bits (true index ^ 0x100 on 9 bits), 16 copies of 8 bytes per entry
+        unsigned char* tab = smem_raw + (kRowsTableAddr - base);
+        static_assert(kRowsThreads == 512, "one table entry per thread");
+        const uint2 v = __ldg(p.table16 + (tid ^ 0x100));
+        const uint4 vv = make_uint4(v.x, v.y, v.x, v.y);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tab + tid * 128 + ((c + tid) & 7) * 16) = vv;
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    {
+        const Pos keep = pf;
+        const int16_t* kq_ = qp; const __half *kx = xp, *kh = hp;
+        pf = pf0;
+        place();
+#pragma unroll
+        for (int i = 0; i < RING; ++i)
+            if (pf.l < p.n_layers) { if (xlive) load_cols(xp, ring[i].x); next(); }
+        pf = keep; qp = kq_; xp = kx; hp = kh;
+    }
+
+    run_corrections<KIND, NB>(p, warp * gridDim.x + blockIdx.x, gridDim.x * kRowsWarps, lane);
+    if constexpr (KIND == EPTQ_E8) asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();                                           // table complete
+
+    const unsigned area = base;                                // fragment buffers / sums over column groups
+    unsigned char* const area_p = smem_raw;
+    unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB));
+    const unsigned my_buf = kq * 2 * kBuf;
+    const unsigned wr_off = my_buf + ((xcol >> 2) & 1) * kHalf + xrow * 32 + (xcol >> 3) * 8 + (xcol & 3) * 2;
+    const unsigned rd_addr = area + my_buf + g * 32 + t * 8;
+    const unsigned lane_tab = 8u * (lane & 15) | kRowsTableAddr;
+    const unsigned tbase = base + e8_table_offset(NB);
+
+    float acc[BT][4][4];
+#pragma unroll
+    for (int i = 0; i < BT; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
+    unsigned par = 0;
+
+    // End of the block's share of a row tile: sum over the column groups, partial sums to scratch, ticket.
+    auto flush = [&]() {
+        const RowsLayer& L = p.L[cur.l];
+        float* red = reinterpret_cast<float*>(area_p) + ctid;
+        __syncthreads();             // fragment buffers are free
+#pragma unroll
+        for (int r = kColGroups - 1; r >= 0; --r) {
+            if (kq == r) {
+#pragma unroll
+                for (int i = 0; i < BT; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+#pragma unroll
+                        for (int c = 0; c < 4; ++c) {
+                            float v = acc[i][j][c];
+                            if (r < kColGroups - 1) v += red[((i * 4 + j) * 4 + c) * 128];
+                            if (r > 0) red[((i * 4 + j) * 4 + c) * 128] = v; else acc[i][j][c] = v;
+                        }
+            }
+            if (r > 0) __syncthreads();
+        }
+        if (kq == 0) {
+            float* dst = p.partial + (static_cast<size_t>(blockIdx.x + L.tile0 + cur.rt) * NB) * kTileOut + (rg * 8 + g) * 8;
+            const float inv = L.x_inv_scale;
+#pragma unroll
+            for (int i = 0; i < BT; ++i)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {                  // batch rows 2t and 2t+1 of the column tile
+                    float v[8];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) { v[2 * j] = acc[i][j][e] * inv; v[2 * j + 1] = acc[i][j][2 + e] * inv; }
+                    if constexpr (NB == 4) {                   // columns 4..7 hold the remainders
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
+                    }
+                    const int b = i * 8 + 2 * t + e;
+                    if ((NB > 4 || t < 2) && b < p.B) {
+                        float4* d4 = reinterpret_cast<float4*>(dst + static_cast<size_t>(b) * kTileOut);
+                        __stcg(d4, make_float4(v[0], v[1], v[2], v[3]));
+                        __stcg(d4 + 1, make_float4(v[4], v[5], v[6], v[7]));
+                    }
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < BT; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[i][j][c] = 0.f;
+        __syncthreads();
+        if (tid == 0) *flag = last_arrival(p, L, cur.rt) ? 1u : 0u;
+        __syncthreads();
+        if (*flag != 0u) finish_tile<NB>(p, L, cur.rt, tid, kRowsThreads);
+    };
+    // Segment after the current one; false when the block's share is done.
+    auto next_segment = [&]() {
+        cur.tile_s0 += p.L[cur.l].ns;
+        if (cur.tile_s0 >= s_end) return false;
+        if (++cur.rt == p.L[cur.l].row_tiles) { cur.rt = 0; ++cur.l; }
+        cur.kend = min(p.L[cur.l].ns, static_cast<int>(s_end - cur.tile_s0));
+        cur.k = kq;
+        return true;
+    };
+
+    auto step = [&](Raw& in) {
+        const uint4 q = in.q;
+        const unsigned qw[4] = {q.x, q.y, q.z, q.w};
+        unsigned ent[8];
+        if constexpr (KIND == EPTQ_E8) {                       // lookups first: some go to L2
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const unsigned w = qw[k] ^ 0x80008000u;
+                ent[2 * k] = e8_fetch<NB>(w & 0xFFFFu, tbase, p.packed);
+                ent[2 * k + 1] = e8_fetch<NB>(w >> 16, tbase, p.packed);
+            }
+        }
+        {
+            const float sc = p.L[cur.l].x_scale;
+            __half hi[XC], lo[XC];
+#pragma unroll
+            for (int e = 0; e < XC; ++e) {
+                const unsigned short xb = static_cast<unsigned short>(in.x[e >> 1] >> (16 * (e & 1)));
+                const unsigned short hb = static_cast<unsigned short>(in.h[e >> 1] >> (16 * (e & 1)));
+                split_half(__half2float(__ushort_as_half(xb)) * (__half2float(__ushort_as_half(hb)) * sc), hi[e], lo[e]);
+            }
+            unsigned char* w = area_p + wr_off + par * kBuf;
+            if constexpr (XC == 4) {
+                *reinterpret_cast<uint2*>(w) = *reinterpret_cast<const uint2*>(hi);
+                *reinterpret_cast<uint2*>(w + kLoPlane) = *reinterpret_cast<const uint2*>(lo);
+            } else if constexpr (XC == 2) {
+                *reinterpret_cast<unsigned*>(w) = *reinterpret_cast<const unsigned*>(hi);
+                *reinterpret_cast<unsigned*>(w + kLoPlane) = *reinterpret_cast<const unsigned*>(lo);
+            } else {
+                *reinterpret_cast<__half*>(w) = hi[0];
+                *reinterpret_cast<__half*>(w + kLoPlane) = lo[0];
+            }
+        }
+        if (pf.l < p.n_layers) {
+            in.q = ldg_once(qp);
+            load_cols(hp, in.h);
+            if (xlive) load_cols(xp, in.x);
+            next();
+        }
+        asm volatile("bar.sync %0, 128;" :: "r"(2 + kq) : "memory");     // the step's fragments are complete
+        const unsigned rd = rd_addr + par * kBuf;
+        par ^= 1;
+        constexpr int PLANES = NB == 4 ? 1 : 2 * BT;           // column tiles: fp16 parts, then remainders
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) {                       // 16 columns: four of this lane's eight
+            uint2 bf[PLANES];
+#pragma unroll
+            for (int i = 0; i < PLANES; ++i) bf[i] = lds64(rd + ks * kHalf + (i % BT) * 256 + (i / BT) * kLoPlane);
+            unsigned c[4][4];                                  // [column][dim pair]
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if constexpr (KIND == EPTQ_E8) {
+                    e8_entry(ent[4 * ks + e], c[e]);
+                } else {
+                    const unsigned v = (e & 1) ? qw[2 * ks + (e >> 1)] >> 16 : qw[2 * ks + (e >> 1)];
+                    const uint2 a = lds64((v & 0xFF80u) | lane_tab);
+                    const uint2 b = lds64(((v << 7) & 0x3F80u) | ((v & 0xC000u) | lane_tab));
+                    c[e][0] = a.x; c[e][1] = a.y; c[e][2] = b.x; c[e][3] = b.y;
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned a[4] = {lo_halves(c[0][j], c[1][j]), hi_halves(c[0][j], c[1][j]),
+                                       lo_halves(c[2][j], c[3][j]), hi_halves(c[2][j], c[3][j])};
+#pragma unroll
+                for (int i = 0; i < PLANES; ++i) mma(acc[i % BT][j], a, bf[i].x, bf[i].y);
+            }
+        }
+    };
+
+    for (bool more = true; more;) {
+#pragma unroll
+        for (int i = 0; i < RING; ++i) {
+            while (more && cur.k >= cur.kend) { flush(); more = next_segment(); }
+            if (!more) break;
+            step(ring[i]);
+            cur.k += kColGroups;
+        }
+    }
+}
+
+struct RowsPlan {
+    unsigned W = 0;
+    int G = 0, tiles = 0, corr_units = 0;
+    size_t bytes = 0;
+};
+
+int rows_of(int B) { return B <= 4 ? 4 : B <= 8 ? 8 : 16; }
+
+bool plan_rows(const EptqLayer* layers, int n, int B, int n_sms, RowsPlan& plan) {
+    if (n < 1 || n > kRowsMaxLayers || n_sms < 1) return false;
+    long long W = 0, tiles = 0;
+    for (int i = 0; i < n; ++i) {
+        const long long rt = (layers[i].M + kTileRows - 1) / kTileRows;
+        tiles += rt;
+        W += rt * (layers[i].N / 32);
+    }
+    if (W < 1 || tiles > kMaxCounters - 1) return false;
+    // A block has at least one step per column group, or the sums over blocks cost more than they spread.
+    const long long G = W / kColGroups < n_sms ? (W / kColGroups > 0 ? W / kColGroups : 1) : n_sms;
+    if (W * G >= (1LL << 32)) return false;
+    plan.W = static_cast<unsigned>(W);
+    plan.G = static_cast<int>(G);
+    plan.tiles = static_cast<int>(tiles);
+    plan.bytes = kPartialOffset + static_cast<size_t>(G + 2 * tiles) * rows_of(B) * kTileOut * sizeof(float);
+    return true;
+}
+
+template <int KIND, int NB, int MAXL>
+int launch_kernel(const RowsArgs<MAXL>& a, int n_sms, cudaStream_t stream) {
+    constexpr int smem = KIND == EPTQ_E8 ? kRowsSmemE8 : kRowsSmemD4;
+    static std::atomic<bool> attr_done[64];       // setting the attribute twice is harmless; the flag itself must not race
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return EPTQ_ERR_LAUNCH;
+    if (!attr_done[dev]) {
+        if (cudaFuncSetAttribute(gemv_rows_kernel<KIND, NB, MAXL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+            return EPTQ_ERR_LAUNCH;
+        attr_done[dev] = true;
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(n_sms);
+    cfg.blockDim = dim3(kRowsThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_rows_kernel<KIND, NB, MAXL>, a);
+    count_launch(EPTQ_KERNEL_GEMV_GROUP);
+    return err == cudaSuccess ? EPTQ_OK : EPTQ_ERR_LAUNCH;
+}
+
+template <int MAXL>
+int launch_sized(const RowsPlan& plan, const EptqLayer* layers, int n, const uint16_t* const* xs, uint16_t* const* ys, int B,
+                 void* workspace, cudaStream_t stream) {
+    const bool e8 = layers[0].quantizer == EPTQ_E8;
+    RowsArgs<MAXL> a;
+    a.table16 = reinterpret_cast<const uint2*>(layers[0].table16);
+    a.packed = e8 ? layers[0].table_packed : nullptr;
+    a.counters = reinterpret_cast<unsigned*>(workspace);
+    a.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kPartialOffset);
+    a.W = plan.W; a.G = plan.G; a.tiles = plan.tiles;
+    a.n_layers = n;
+    a.B = B;
+    int step0 = 0, tile0 = 0, corr0 = 0;
+    for (int i = 0; i < n; ++i) {
+        const EptqLayer& L = layers[i];
+        RowsLayer& R = a.L[i];
+        if (xs[i] == nullptr || ys[i] == nullptr) return EPTQ_ERR_NULL;
+        if (!aligned16(xs[i]) || !aligned16(ys[i])) return EPTQ_ERR_ALIGN;
+        R.Q = L.Q;
+        R.g = reinterpret_cast<const __half*>(L.g);
+        R.h = reinterpret_cast<const __half*>(L.h);
+        R.x = reinterpret_cast<const __half*>(xs[i]);
+        R.O_vals = reinterpret_cast<const __half*>(L.O_vals);
+        R.O_col = L.O_col;
+        R.O_row_ptr = L.O_row_ptr;
+        R.bias = reinterpret_cast<const __half*>(L.bias);
+        R.y = reinterpret_cast<__half*>(ys[i]);
+        R.M = L.M; R.N = L.N;
+        R.ns = L.N / 32;
+        R.row_tiles = (L.M + kTileRows - 1) / kTileRows;
+        R.step0 = step0; R.tile0 = tile0; R.corr0 = corr0;
+        R.corr_tile = L.n_masked != 0 ? kCorrPerTile : 0;      // -1 (count unknown): the row pointers carry it
+        int e = 0;
+        std::frexp(L.h_absmax, &e);            // h_absmax = m * 2^e, m in [0.5, 1)  =>  2^-e <= 1/h_absmax
+        R.x_scale = std::ldexp(1.0f, -e);
+        R.x_inv_scale = std::ldexp(1.0f, e) * (e8 ? L.table_packed_scale : 1.0f);
+        step0 += R.row_tiles * R.ns;
+        tile0 += R.row_tiles;
+        corr0 += R.row_tiles * R.corr_tile;
+    }
+    a.corr_units = corr0;
+    switch (rows_of(B)) {
+        case 4: return e8 ? launch_kernel<EPTQ_E8, 4>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 4>(a, plan.G, stream);
+        case 8: return e8 ? launch_kernel<EPTQ_E8, 8>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 8>(a, plan.G, stream);
+        default: return e8 ? launch_kernel<EPTQ_E8, 16>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 16>(a, plan.G, stream);
+    }
+}
+
+}  // namespace
+
+// Scratch of the one-pass launch, 0 if the shapes do not fit its plan.  The layers are ones group_gemv_supported takes.
+size_t rows_workspace_bytes(const EptqLayer* layers, int n, int B, int n_sms) {
+    RowsPlan plan;
+    return plan_rows(layers, n, B, n_sms, plan) ? (plan.bytes + 255) & ~static_cast<size_t>(255) : 0;
+}
+
+int launch_gemv_rows(const EptqLayer* layers, int n, const uint16_t* const* xs, uint16_t* const* ys, int B, int n_sms,
+                     void* workspace, cudaStream_t stream) {
+    RowsPlan plan;
+    if (!plan_rows(layers, n, B, n_sms, plan)) return EPTQ_ERR_UNSUPPORTED;
+    return n <= kRowsFewLayers ? launch_sized<kRowsFewLayers>(plan, layers, n, xs, ys, B, workspace, stream)
+                               : launch_sized<kRowsMaxLayers>(plan, layers, n, xs, ys, B, workspace, stream);
+}
+
+}  // namespace eptq

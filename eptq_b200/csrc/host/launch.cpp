@@ -56,19 +56,33 @@ bool is_current(const LayerHandle* h) {
     return true;
 }
 
-// One zero-filled scratch tensor per (device, stream), grown on demand; only touched with the GIL held.
-std::map<std::pair<int, int64_t>, at::Tensor>& scratch_map() {
-    static auto* m = new std::map<std::pair<int, int64_t>, at::Tensor>();         // never destroyed: no CUDA calls at exit
+// One zero-filled scratch tensor per (device, stream), grown on demand; only touched with the GIL held.  A CUDA graph
+// keeps the addresses it was captured with, so a tensor handed out during a capture is kept when a larger one
+// replaces it.
+struct Scratch { at::Tensor t; bool captured = false; };
+std::map<std::pair<int, int64_t>, Scratch>& scratch_map() {
+    static auto* m = new std::map<std::pair<int, int64_t>, Scratch>();            // never destroyed: no CUDA calls at exit
     return *m;
 }
 
+std::vector<std::pair<int, at::Tensor>>& kept_scratch() {
+    static auto* v = new std::vector<std::pair<int, at::Tensor>>();
+    return *v;
+}
+
 const at::Tensor& scratch_for(int device, const c10::cuda::CUDAStream& stream, size_t bytes) {
-    at::Tensor& t = scratch_map()[{device, static_cast<int64_t>(reinterpret_cast<intptr_t>(stream.stream()))}];
-    if (!t.defined() || static_cast<size_t>(t.numel()) < bytes) {
+    Scratch& s = scratch_map()[{device, static_cast<int64_t>(reinterpret_cast<intptr_t>(stream.stream()))}];
+    if (!s.t.defined() || static_cast<size_t>(s.t.numel()) < bytes) {
+        if (s.captured) kept_scratch().emplace_back(device, std::move(s.t));
         const int64_t n = static_cast<int64_t>(bytes > kMinScratch ? bytes : kMinScratch);
-        t = at::zeros({n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+        s.t = at::zeros({n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
+        s.captured = false;
     }
-    return t;
+    if (!s.captured) {
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        s.captured = cudaStreamIsCapturing(stream.stream(), &st) == cudaSuccess && st != cudaStreamCaptureStatusNone;
+    }
+    return s.t;
 }
 
 bool fail(int status, const char* what) {
@@ -284,9 +298,13 @@ PyObject* scratch_of_device(PyObject*, PyObject* const* a, Py_ssize_t n) {
     if (PyErr_Occurred()) return nullptr;
     PyObject* out = PyList_New(0);
     if (out == nullptr) return nullptr;
-    for (auto& kv : scratch_map()) {
-        if (kv.first.first != device) continue;
-        PyObject* t = THPVariable_Wrap(kv.second);
+    std::vector<at::Tensor> all;
+    for (const auto& kv : scratch_map())
+        if (kv.first.first == device) all.push_back(kv.second.t);
+    for (const auto& kv : kept_scratch())
+        if (kv.first == device) all.push_back(kv.second);
+    for (const at::Tensor& s : all) {
+        PyObject* t = THPVariable_Wrap(s);
         if (t == nullptr || PyList_Append(out, t) != 0) { Py_XDECREF(t); Py_DECREF(out); return nullptr; }
         Py_DECREF(t);
     }

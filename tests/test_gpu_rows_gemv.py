@@ -1,0 +1,75 @@
+"""One pass over the weights for 3 to 16 batch rows (gemv_rows_kernel) against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from eptq_b200 import _lib
+from eptq_b200.kernels.linear import EPTQLinear, forward_group
+from eptq_b200.synthetic import make_activations, make_layer
+from tests import util
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+TABLES = {"e8_d4": oracle.d4_table(1.75), "e8_lattice": oracle.e8_table(1.6)}
+
+
+def layers_of(kind, shapes, fractions=(0.004, 0.0, 0.02)):
+    qds = [make_layer(o, i, seed=7 * k + o + i, outlier_frac=fractions[k % len(fractions)], bias=(k % 2 == 0))
+           for k, (o, i) in enumerate(shapes)]
+    return qds, [EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV) for qd in qds]
+
+
+def check(kind, qds, xs, ys):
+    for qd, x, y in zip(qds, xs, ys):
+        W16 = oracle.dequantize_layer(util.qld_arrays(qd), TABLES[kind])
+        ref = oracle.linear_reference(x.numpy(), W16, None if qd.bias is None else qd.bias.numpy())
+        for b in range(x.shape[0]):                     # row by row: rows may differ in scale
+            assert util.max_rel_err(y[b].float().cpu().numpy(), ref[b]) <= util.REL_TOL
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("batch", [3, 4, 5, 8, 9, 16])
+def test_rows_match_oracle(kind, batch):
+    # shares that begin and end inside row tiles, ragged row counts, one row, one 32-column step, layers without
+    # critical blocks between layers with them
+    shapes = [(1288, 2752), (264, 4096), (8, 32), (4096, 1056), (40, 96)]
+    qds, lins = layers_of(kind, shapes)
+    xs = [make_activations(batch, i, seed=61 + k) * (10.0 ** (k % 3 - 1)) for k, (_, i) in enumerate(shapes)]
+    for _ in range(2):                                  # the scratch is left clean
+        ys = forward_group(lins, [x.to(DEV) for x in xs])
+        check(kind, qds, xs, ys)
+    first = forward_group(lins, [x.to(DEV) for x in xs])
+    again = forward_group(lins, [x.to(DEV) for x in xs])
+    assert all(torch.equal(a, b) for a, b in zip(first, again))          # partials are added in a fixed order
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_rows_many_layers_and_all_markers(kind):
+    qds, lins = layers_of(kind, [(64, 64 + 32 * (k % 5)) for k in range(32)])
+    qds[3] = make_layer(64, qds[3].Q.shape[1], seed=5, outlier_frac=1.1)                 # nothing but critical blocks
+    lins[3] = EPTQLinear.from_quantized_data(qds[3], torch.from_numpy(TABLES[kind]), kind).to(DEV)
+    lins[3]._codebook = lins[0]._codebook
+    lins[3]._codebook32 = lins[0]._codebook32
+    xs = [make_activations(6, qd.Q.shape[1], seed=9 + k) for k, qd in enumerate(qds)]
+    check(kind, qds, xs, forward_group(lins, [x.to(DEV) for x in xs]))
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_small_scratch_takes_passes_of_two_rows(kind):
+    """A caller whose scratch holds no partial sums still gets its result."""
+    import ctypes as C
+    qds, lins = layers_of(kind, [(4096, 1024), (1024, 1024)])
+    x = make_activations(7, 1024, seed=3)
+    xd = x.to(DEV)
+    lib = _lib.load()
+    descs = (_lib.EptqLayer * 2)(*[lin.descriptor() for lin in lins])
+    assert lib.eptq_group_workspace_bytes(C.byref(descs), 2, 7) > 1 << 20
+    ws = torch.zeros(1 << 20, dtype=torch.uint8, device=DEV)
+    ys = [torch.empty((7, lin.out_features), dtype=torch.float16, device=DEV) for lin in lins]
+    xp = (C.c_void_p * 2)(xd.data_ptr(), xd.data_ptr())
+    yp = (C.c_void_p * 2)(*[y.data_ptr() for y in ys])
+    st = lib.eptq_linear_forward_group(C.byref(descs), 2, xp, yp, 7, ws.data_ptr(), ws.numel(),
+                                       torch.cuda.current_stream().cuda_stream)
+    assert st == 0
+    check(kind, qds, [x, x], ys)
