@@ -22,7 +22,8 @@
 //
 // Critical blocks: while the table arrives, the warps of the launch walk the CSR tables in units of 4 Q rows (at most a
 // unit or two per warp for the fractions in use) and store sum (O - code[65535])*h*x to a slot of their own that the
-// last arrival adds.  Dedicated warps for it would leave 96 registers a thread, and the main loop then spills: to L2,
+// last arrival adds; what does not need x is read before the dependency wait, and the ticket is looked at behind the main
+// loop (4096 x 4096 E8-D4: 14.1 -> 13.3 us at 4 rows, 16.1 -> 15.2 at 8).  Dedicated warps for it would leave 96 registers a thread, and the main loop then spills: to L2,
 // since nearly all of L1 is shared memory (4096 x 4096 E8-D4, 16 rows: 60.3 against 23.7 us a call).
 
 #include <atomic>
@@ -164,33 +165,26 @@ __device__ __forceinline__ void finish_tile(const RowsArgs<MAXL>& p, const RowsL
         const int b = i / (kTileOut / 4), q = i % (kTileOut / 4);
         if (rt * kTileRows + (q >> 1) >= L.M) continue;
         const size_t off = static_cast<size_t>(b) * kTileOut + q * 4;
-        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
-        int k = 0;
-        for (; k + 4 <= last - first + 1; k += 4) {                     // four loads in flight
-            float4 v[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) v[j] = __ldcg(reinterpret_cast<const float4*>(parts + (k + j) * slot + off));
-#pragma unroll
-            for (int j = 0; j < 4; ++j) { s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w; }
-        }
-        for (; k <= last - first; ++k) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(parts + k * slot + off));
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-        }
-        if (corr != nullptr) {
-            const float4 v = __ldcg(reinterpret_cast<const float4*>(corr + off));
-            s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-        }
         const int o = rt * kTileOut + q * 4;
         const uint2 graw = __ldg(reinterpret_cast<const uint2*>(L.g + o));
+        uint2 braw = make_uint2(0, 0);
+        if (L.bias != nullptr) braw = __ldg(reinterpret_cast<const uint2*>(L.bias + o));
+        float4 cv = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (corr != nullptr) cv = __ldcg(reinterpret_cast<const float4*>(corr + off));
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k <= last - first; k += 8) {                     // eight loads in flight
+            float4 v[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+                v[j] = k + j <= last - first ? __ldcg(reinterpret_cast<const float4*>(parts + (k + j) * slot + off)) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) { s.x += v[j].x; s.y += v[j].y; s.z += v[j].z; s.w += v[j].w; }
+        }
+        s.x += cv.x; s.y += cv.y; s.z += cv.z; s.w += cv.w;
         const float2 g01 = __half22float2(*reinterpret_cast<const __half2*>(&graw.x));
         const float2 g23 = __half22float2(*reinterpret_cast<const __half2*>(&graw.y));
-        float2 b01 = make_float2(0.f, 0.f), b23 = make_float2(0.f, 0.f);
-        if (L.bias != nullptr) {
-            const uint2 braw = __ldg(reinterpret_cast<const uint2*>(L.bias + o));
-            b01 = __half22float2(*reinterpret_cast<const __half2*>(&braw.x));
-            b23 = __half22float2(*reinterpret_cast<const __half2*>(&braw.y));
-        }
+        const float2 b01 = __half22float2(*reinterpret_cast<const __half2*>(&braw.x));
+        const float2 b23 = __half22float2(*reinterpret_cast<const __half2*>(&braw.y));
         const __half2 o01 = __floats2half2_rn(fmaf(s.x, g01.x, b01.x), fmaf(s.y, g01.y, b01.y));
         const __half2 o23 = __floats2half2_rn(fmaf(s.z, g23.x, b23.x), fmaf(s.w, g23.y, b23.y));
         uint2 ov;
@@ -209,9 +203,35 @@ __device__ __forceinline__ bool last_arrival(const RowsArgs<MAXL>& p, const Rows
     return ticket == static_cast<unsigned>(n + L.corr_tile) - 1u;
 }
 
-// Correction units cw, cw + n_warps, ...: 4 Q rows each, 8 lanes per row, four batch rows at a time.
+// A unit of corrections: 4 Q rows, 8 lanes per row.  `lo`, `hi`: this lane's row in the CSR tables; col, h, O: its first
+// critical block, read ahead.
+struct CorrUnit {
+    int l, qt, lo, hi, col;
+    float h;
+    uint4 O;
+};
+template <int MAXL>
+__device__ __forceinline__ CorrUnit corr_begin(const RowsArgs<MAXL>& p, int u, int lane) {
+    CorrUnit c;
+    c.l = 0;
+    while (c.l + 1 < p.n_layers && p.L[c.l + 1].corr0 <= u) ++c.l;     // layers without units share their successor's corr0
+    const RowsLayer& L = p.L[c.l];
+    c.qt = u - L.corr0;
+    const int row = c.qt * 4 + (lane >> 3);
+    c.lo = c.hi = 0;
+    if (row < L.M) { c.lo = __ldg(L.O_row_ptr + row); c.hi = __ldg(L.O_row_ptr + row + 1); }
+    c.col = 0; c.h = 0.f; c.O = make_uint4(0, 0, 0, 0);
+    const int i = c.lo + (lane & 7);
+    if (i < c.hi) {
+        c.col = __ldg(L.O_col + i);
+        c.O = ldg128(L.O_vals + static_cast<size_t>(i) * 8);
+        c.h = __half2float(__ldg(L.h + c.col));
+    }
+    return c;
+}
+// Four batch rows at a time; stores the sums and takes the tile's ticket.  Returns whether it was the last.
 template <int KIND, int NB, int MAXL>
-__device__ void run_corrections(const RowsArgs<MAXL>& p, int cw, int n_warps, int lane) {
+__device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrUnit& c, int lane) {
     float cstar[4] = {0.f, 0.f, 0.f, 0.f};                     // what the main loop adds for a marker (E8: zero)
     if (KIND == EPTQ_E8D4) {
         const uint2 raw = __ldg(p.table16 + 511);
@@ -219,57 +239,53 @@ __device__ void run_corrections(const RowsArgs<MAXL>& p, int cw, int n_warps, in
         const float2 c23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
         cstar[0] = c01.x; cstar[1] = c01.y; cstar[2] = c23.x; cstar[3] = c23.y;
     }
-    int l = 0;
-    for (int u = cw; u < p.corr_units; u += n_warps) {
-        while (l + 1 < p.n_layers && p.L[l + 1].corr0 <= u) ++l;     // layers without units share their successor's corr0
-        const RowsLayer& L = p.L[l];
-        const int qt = u - L.corr0, rt = qt / kCorrPerTile;
-        const int row = qt * 4 + (lane >> 3), sub = lane & 7;
-        int lo = 0, hi = 0;
-        if (row < L.M) { lo = __ldg(L.O_row_ptr + row); hi = __ldg(L.O_row_ptr + row + 1); }
-        float* dst = p.partial + (static_cast<size_t>(p.G + p.tiles + L.tile0 + rt) * NB) * kTileOut + ((qt % kCorrPerTile) * 4 + (lane >> 3)) * 8;
-        for (int b0 = 0; b0 < p.B; b0 += 4) {
-            float acc[4][8];
+    const RowsLayer& L = p.L[c.l];
+    const int rt = c.qt / kCorrPerTile, sub = lane & 7;
+    float* dst = p.partial + (static_cast<size_t>(p.G + p.tiles + L.tile0 + rt) * NB) * kTileOut + ((c.qt % kCorrPerTile) * 4 + (lane >> 3)) * 8;
+    for (int b0 = 0; b0 < p.B; b0 += 4) {
+        float acc[4][8];
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+#pragma unroll
+            for (int k = 0; k < 8; ++k) acc[b][k] = 0.f;
+        int col = c.col;
+        float hv = c.h;
+        uint4 ov = c.O;
+        for (int i = c.lo + sub; i < c.hi;) {
+            float o8[8], xv[4];
+            unpack8(ov, o8);
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                xv[b] = b0 + b < p.B ? hv * __half2float(__ldg(L.x + static_cast<size_t>(b0 + b) * L.N + col)) : 0.f;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[b][k] = 0.f;
-            for (int i = lo + sub; i < hi; i += 8) {
-                const int col = __ldg(L.O_col + i);
-                const float hv = __half2float(__ldg(L.h + col));
-                float o8[8];
-                unpack8(ldg128(L.O_vals + static_cast<size_t>(i) * 8), o8);
-                float xv[4];
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-                    xv[b] = b0 + b < p.B ? hv * __half2float(__ldg(L.x + static_cast<size_t>(b0 + b) * L.N + col)) : 0.f;
-#pragma unroll
-                for (int b = 0; b < 4; ++b)
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) acc[b][k] = fmaf(o8[k] - cstar[k & 3], xv[b], acc[b][k]);
-            }
-            __syncwarp();
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {
-                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 1);
-                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 2);
-                    acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 4);
-                }
-                if (sub == 0 && b0 + b < p.B) {
-                    float4* d4 = reinterpret_cast<float4*>(dst + static_cast<size_t>(b0 + b) * kTileOut);
-                    __stcg(d4, make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]));
-                    __stcg(d4 + 1, make_float4(acc[b][4], acc[b][5], acc[b][6], acc[b][7]));
-                }
+                for (int k = 0; k < 8; ++k) acc[b][k] = fmaf(o8[k] - cstar[k & 3], xv[b], acc[b][k]);
+            i += 8;
+            if (i < c.hi) {
+                col = __ldg(L.O_col + i);
+                ov = ldg128(L.O_vals + static_cast<size_t>(i) * 8);
+                hv = __half2float(__ldg(L.h + col));
             }
         }
         __syncwarp();
-        int mine = 0;
-        if (lane == 0) mine = last_arrival(p, L, rt);
-        if (__shfl_sync(0xffffffffu, mine, 0)) finish_tile<NB>(p, L, rt, lane, 32);
-        __syncwarp();
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 1);
+                acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 2);
+                acc[b][k] += __shfl_xor_sync(0xffffffffu, acc[b][k], 4);
+            }
+            if (sub == 0 && b0 + b < p.B) {
+                float4* d4 = reinterpret_cast<float4*>(dst + static_cast<size_t>(b0 + b) * kTileOut);
+                __stcg(d4, make_float4(acc[b][0], acc[b][1], acc[b][2], acc[b][3]));
+                __stcg(d4 + 1, make_float4(acc[b][4], acc[b][5], acc[b][6], acc[b][7]));
+            }
+        }
     }
+    __syncwarp();
+    return lane == 0 && last_arrival(p, L, rt);
 }
 
 template <int KIND, int NB, int MAXL>
@@ -371,6 +387,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
 #pragma unroll
         for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tab + tid * 128 + ((c + tid) & 7) * 16) = vv;
     }
+    const int unit0 = warp * gridDim.x + blockIdx.x, unit_step = gridDim.x * kRowsWarps;
+    CorrUnit corr = {};
+    if (unit0 < p.corr_units) corr = corr_begin(p, unit0, lane);
     asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         const Pos keep = pf;
@@ -383,7 +402,16 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         pf = keep; qp = kq_; xp = kx; hp = kh;
     }
 
-    run_corrections<KIND, NB>(p, warp * gridDim.x + blockIdx.x, gridDim.x * kRowsWarps, lane);
+    // The first unit's ticket is looked at behind the main loop (its round trip costs nothing there).
+    bool corr_last = false;
+    if (unit0 < p.corr_units) corr_last = corr_finish<KIND, NB>(p, corr, lane);
+    const int corr_l = corr.l, corr_rt = corr.qt / kCorrPerTile;
+    for (int u = unit0 + unit_step; u < p.corr_units; u += unit_step) {
+        const CorrUnit c = corr_begin(p, u, lane);
+        const bool last = corr_finish<KIND, NB>(p, c, lane);
+        if (__any_sync(0xffffffffu, last)) finish_tile<NB>(p, p.L[c.l], c.qt / kCorrPerTile, lane, 32);
+        __syncwarp();
+    }
     if constexpr (KIND == EPTQ_E8) asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();                                           // table complete
 
@@ -469,18 +497,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         return true;
     };
 
-    auto step = [&](Raw& in) {
+    // E8 lookups run one step ahead: a seventh of them goes to L2, and waiting for those was half of a step (gate/up of a
+    // 7B model: 48.9 -> 36.1 us at 4 rows, 57.4 -> 37.9 at 8, 64.5 -> 48.9 at 16).
+    unsigned ent[8];
+    auto lookup = [&](const uint4& q, unsigned (&e)[8]) {
+        const unsigned w[4] = {q.x ^ 0x80008000u, q.y ^ 0x80008000u, q.z ^ 0x80008000u, q.w ^ 0x80008000u};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            e[2 * k] = e8_fetch<NB>(w[k] & 0xFFFFu, tbase, p.packed);
+            e[2 * k + 1] = e8_fetch<NB>(w[k] >> 16, tbase, p.packed);
+        }
+    };
+    if constexpr (KIND == EPTQ_E8) lookup(ring[0].q, ent);
+
+    auto step = [&](Raw& in, const Raw& following) {
         const uint4 q = in.q;
         const unsigned qw[4] = {q.x, q.y, q.z, q.w};
-        unsigned ent[8];
-        if constexpr (KIND == EPTQ_E8) {                       // lookups first: some go to L2
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const unsigned w = qw[k] ^ 0x80008000u;
-                ent[2 * k] = e8_fetch<NB>(w & 0xFFFFu, tbase, p.packed);
-                ent[2 * k + 1] = e8_fetch<NB>(w >> 16, tbase, p.packed);
-            }
-        }
         {
             const float sc = p.L[cur.l].x_scale;
             __half hi[XC], lo[XC];
@@ -511,6 +543,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         asm volatile("bar.sync %0, 128;" :: "r"(2 + kq) : "memory");     // the step's fragments are complete
         const unsigned rd = rd_addr + par * kBuf;
         par ^= 1;
+        unsigned ahead[8];
+        if constexpr (KIND == EPTQ_E8) lookup(following.q, ahead);       // behind the last step: zeros, a valid index
         constexpr int PLANES = NB == 4 ? 1 : 2 * BT;           // column tiles: fp16 parts, then remainders
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {                       // 16 columns: four of this lane's eight
@@ -537,6 +571,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
                 for (int i = 0; i < PLANES; ++i) mma(acc[i % BT][j], a, bf[i].x, bf[i].y);
             }
         }
+        if constexpr (KIND == EPTQ_E8) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) ent[e] = ahead[e];
+        }
     };
 
     for (bool more = true; more;) {
@@ -544,10 +582,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         for (int i = 0; i < RING; ++i) {
             while (more && cur.k >= cur.kend) { flush(); more = next_segment(); }
             if (!more) break;
-            step(ring[i]);
+            step(ring[i], ring[(i + 1) % RING]);
             cur.k += kColGroups;
         }
     }
+    if (__any_sync(0xffffffffu, corr_last)) finish_tile<NB>(p, p.L[corr_l], corr_rt, lane, 32);
 }
 
 struct RowsPlan {
