@@ -28,7 +28,9 @@ int launch_gemv_mma(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B,
 bool gemm_supported(const EptqLayer& L, int T);
 int launch_gemm_tcgen05(const EptqLayer& L, const uint16_t* x, uint16_t* y, int T, int* status, cudaStream_t stream);
 bool gemm_ws_supported(const EptqLayer& L, const void* x, int T);
-int launch_gemm_tcgen05_ws(const EptqLayer& L, const uint16_t* x, uint16_t* y, int T, int* status, cudaStream_t stream);
+int launch_gemm_tcgen05_ws(const EptqLayer& L, const uint16_t* x, uint16_t* y, int T, void* workspace, size_t workspace_bytes,
+                           cudaStream_t stream);
+size_t gemm_ws_partial_bytes(int kind, int M, int N, int T);
 bool gemm_dense_supported(int T, int N, const void* x, const void* y, const void* bias);
 int launch_gemm_dense(const uint16_t* W16, const uint16_t* x, uint16_t* y, const uint16_t* bias, int T, int out, int N,
                       int* status, cudaStream_t stream);
@@ -88,7 +90,7 @@ int forward_checked(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B,
             return launch_gemm_dense(W16, x, y, L.bias, B, 8 * L.M, L.N, status, static_cast<cudaStream_t>(stream));
         }
         if (gemm_ws_supported(L, x, B))
-            return launch_gemm_tcgen05_ws(L, x, y, B, status, static_cast<cudaStream_t>(stream));
+            return launch_gemm_tcgen05_ws(L, x, y, B, workspace, workspace_bytes, static_cast<cudaStream_t>(stream));
         return launch_gemm_tcgen05(L, x, y, B, status, static_cast<cudaStream_t>(stream));
     }
     if (stream_gemv_supported(&L, 1, B) && aligned16(y) && workspace != nullptr && workspace_bytes >= kPartialOffset) {
@@ -193,9 +195,11 @@ size_t eptq_workspace_bytes(int M, int N, int B) {
 
 size_t eptq_layer_workspace_bytes(const EptqLayer* layer, int B) {
     if (layer == nullptr || B <= 0) return 0;
-    // Above the GEMV batch limit a layer the tensor-core GEMM takes needs the counter block only.
+    // Above the GEMV batch limit a layer the tensor-core GEMM takes needs the counter block only; more is for the
+    // reconstructed weight or for the partial sums of K ranges.
     if (B > kGemmMinBatch && gemm_supported(*layer, B))
-        return kPartialOffset + (B >= kDenseMinTokens ? dense_weight_bytes(layer->M, layer->N) : 0);
+        return kPartialOffset + (B >= kDenseMinTokens ? dense_weight_bytes(layer->M, layer->N)
+                                                      : (gemm_ws_partial_bytes(layer->quantizer, layer->M, layer->N, B) + 255) & ~static_cast<size_t>(255));
     return eptq_workspace_bytes(layer->M, layer->N, B);
 }
 

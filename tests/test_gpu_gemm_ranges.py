@@ -1,0 +1,36 @@
+"""Tensor-core GEMM over K ranges, its index ring and its look-ahead for critical blocks, against the oracle."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from eptq_b200.kernels.linear import EPTQLinear
+from eptq_b200.synthetic import make_activations, make_layer
+from tests import util
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+TABLES = {"e8_d4": oracle.d4_table(1.75), "e8_lattice": oracle.e8_table(1.6)}
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("out,inn,tokens,qb,frac", [
+    (1024, 4096, 17, 0, 0.004),          # many ranges, a mostly empty token tile
+    (264, 1096, 129, 0, 0.02),           # ragged rows, a last chunk of 8 columns
+    (128, 64, 33, 0, 0.3),               # one chunk, one range
+    (1024, 2056, 300, 128, 0.004),       # group scales shared by a tile
+    (1024, 2056, 100, 64, 0.02),         # group scales that change inside a tile
+    (136, 520, 513, 0, 1.1),             # nothing but critical blocks
+])
+def test_ranges_match_oracle(kind, out, inn, tokens, qb, frac):
+    qd = make_layer(out, inn, seed=out + inn + tokens, outlier_frac=frac, bias=(tokens % 2 == 1), qb_size=qb or None)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV)
+    x = make_activations(tokens, inn, seed=tokens)
+    W16 = oracle.dequantize_layer(util.qld_arrays(qd), TABLES[kind])
+    ref = oracle.linear_reference(x.numpy(), W16, None if qd.bias is None else qd.bias.numpy())
+    xd = x.to(DEV)
+    y = lin(xd)
+    assert util.max_rel_err(y.float().cpu().numpy(), ref) <= util.REL_TOL
+    assert torch.equal(lin(xd), y)                       # ranges are added in a fixed order, the scratch is left clean
+    W = lin.dequantize()
+    assert np.array_equal(W.cpu().numpy().view(np.uint16), np.asarray(W16).view(np.uint16))     # bit-exact
