@@ -38,6 +38,9 @@ bool group_gemv_supported(const EptqLayer* layers, int n, int B);
 size_t group_workspace_bytes(const EptqLayer* layers, int n, int B, int n_sms);
 int launch_gemv_group(const EptqLayer* layers, int n, const EptqFusion* fusions, const uint16_t* const* xs,
                       uint16_t* const* ys, int B, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+size_t rows_workspace_bytes(const EptqLayer* layers, int n, int B, int n_sms);
+bool rows_scaled_supported(const EptqLayer& L, int B);
+int launch_gemv_rows_scaled(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B, int n_sms, void* workspace, cudaStream_t stream);
 bool stream_gemv_supported(const EptqLayer* layers, int n, int B);
 int launch_gemv_stream(const EptqLayer* layers, int n, const EptqFusion* fusions, const int* phases,
                        const uint16_t* const* xs, uint16_t* const* ys, int B, void* workspace, size_t workspace_bytes,
@@ -100,6 +103,11 @@ int forward_checked(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B,
     }
     // The E8 variant copies 219 KB of table into every block: not worth it for a small layer.
     const bool big_enough = L.quantizer != EPTQ_E8 || static_cast<long long>(L.M) * L.N >= (1LL << 20);
+    if (big_enough && L.S_group != nullptr && rows_scaled_supported(L, B) && aligned16(y)) {
+        const size_t need = rows_workspace_bytes(&L, 1, 4, kSms);
+        if (need != 0 && workspace != nullptr && workspace_bytes >= need)
+            return launch_gemv_rows_scaled(L, x, y, B, kSms, workspace, static_cast<cudaStream_t>(stream));
+    }
     if (big_enough && group_gemv_supported(&L, 1, B) && aligned16(y)) {
         const uint16_t* xs[1] = {x};
         uint16_t* ys[1] = {y};
@@ -200,7 +208,12 @@ size_t eptq_layer_workspace_bytes(const EptqLayer* layer, int B) {
     if (B > kGemmMinBatch && gemm_supported(*layer, B))
         return kPartialOffset + (B >= kDenseMinTokens ? dense_weight_bytes(layer->M, layer->N)
                                                       : (gemm_ws_partial_bytes(layer->quantizer, layer->M, layer->N, B) + 255) & ~static_cast<size_t>(255));
-    return eptq_workspace_bytes(layer->M, layer->N, B);
+    size_t bytes = eptq_workspace_bytes(layer->M, layer->N, B);
+    if (rows_scaled_supported(*layer, B)) {
+        const size_t rows = rows_workspace_bytes(layer, 1, 4, kSms);
+        if (rows > bytes) bytes = rows;
+    }
+    return bytes;
 }
 
 size_t eptq_group_workspace_bytes(const EptqLayer* layers, int n_layers, int B) {

@@ -16,6 +16,7 @@
 namespace eptq {
 
 constexpr unsigned kMarkerIndex = 65535u;   // codebook index that marks a critical block
+constexpr int kSms = 148;                   // SMs of the GPU this library is built for
 constexpr int kMaxSplits = 16;              // column splits a GEMV may use (sizes the scratch)
 constexpr int kRowsPerCta = 8;              // Q rows (groups of 8 outputs) per SIMT GEMV block
 

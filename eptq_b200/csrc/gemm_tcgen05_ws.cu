@@ -549,7 +549,6 @@ int launch_ws_shape(int tm, const CUtensorMap& tmap, const CUtensorMap& tmap_q, 
     }
 }
 
-constexpr int kSms = 148;
 int tile_tokens(int T) { return T <= 128 ? 128 : T <= 256 ? 256 : 512; }
 int tile_count(int M, int T) { return ((8 * M + kOutTile - 1) / kOutTile) * ((T + tile_tokens(T) - 1) / tile_tokens(T)); }
 size_t split_bytes(int M, int T, int splits) {

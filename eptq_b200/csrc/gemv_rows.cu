@@ -20,6 +20,11 @@
 // the block's partial sums go to scratch with plain stores; the block (or, for a unit of corrections, warp) that takes the last
 // ticket of a row tile adds the partials in block order, so results do not depend on arrival order.
 //
+// Group scales (SCALED; one layer, passes of 4 rows): the scale of a row group's 64 outputs multiplies x*h before the split,
+// so the four warps of a column group need different fragments and each converts its own (4 values a lane and step).
+// Taken for qb_size % 64 == 0; the SIMT kernel, which multiplies in its inner loop, stays for the rest
+// (14336 x 4096 E8-D4, scales per 128 rows, 1 row: 34.8 -> 19.5 us).
+//
 // Critical blocks: while the table arrives, the warps of the launch walk the CSR tables in units of 4 Q rows (at most a
 // unit or two per warp for the fractions in use) and store sum (O - code[65535])*h*x to a slot of their own that the
 // last arrival adds; what does not need x is read before the dependency wait, and the ticket is looked at behind the main
@@ -53,9 +58,10 @@ constexpr int kRowsSmemE8 = 232448;                             // the most a bl
 constexpr unsigned kCtrlBytes = 64;
 
 // Fragment buffers ([column group][2][hi, lo][NB rows][32 columns] fp16), reused for the sum over column groups.
-__host__ __device__ constexpr unsigned area_bytes(int nb) { return nb == 16 ? 16384u : 8192u; }
-__host__ __device__ constexpr unsigned e8_table_offset(int nb) { return area_bytes(nb) + kCtrlBytes; }
-__host__ __device__ constexpr unsigned e8_resident(int nb) { return (kRowsSmemE8 - e8_table_offset(nb)) / 4; }
+// With group scales every warp has its own buffers.
+__host__ __device__ constexpr unsigned area_bytes(int nb, bool scaled) { return nb == 16 || scaled ? 16384u : 8192u; }
+__host__ __device__ constexpr unsigned e8_table_offset(int nb, bool scaled) { return area_bytes(nb, scaled) + kCtrlBytes; }
+__host__ __device__ constexpr unsigned e8_resident(int nb, bool scaled) { return (kRowsSmemE8 - e8_table_offset(nb, scaled)) / 4; }
 
 struct RowsLayer {
     const int16_t* Q;
@@ -74,7 +80,9 @@ struct RowsLayer {
     int ns;                 // steps per row tile = N / 32
     int row_tiles;          // ceil(M / 32)
     int corr_tile;          // correction units per row tile: 8, or 0 for a layer without critical blocks
-    float x_scale;          // power of two, <= 1 / max|h|
+    int qb_rows;            // Q rows per scale group, 0 without group scales
+    const __half* S;
+    float x_scale;          // power of two, <= 1 / max|h| (/ max|S|)
     float x_inv_scale;
 };
 
@@ -130,7 +138,7 @@ __device__ __forceinline__ void e8_entry(unsigned e, unsigned (&r)[4]) {
         r[i] = *reinterpret_cast<const unsigned*>(&v);
     }
 }
-template <int NB>
+template <int NB, bool SCALED>
 __device__ __forceinline__ unsigned e8_fetch(unsigned u, unsigned tbase, const unsigned* packed) {
     unsigned v;
     asm volatile("{\n\t.reg .pred p;\n\t.reg .u64 ga;\n\t.reg .u32 sa;\n\t"
@@ -139,7 +147,7 @@ __device__ __forceinline__ unsigned e8_fetch(unsigned u, unsigned tbase, const u
                  "mad.lo.u32 sa, %1, 4, %4;\n\t"
                  "@p ld.global.nc.u32 %0, [ga];\n\t"
                  "@!p ld.shared.u32 %0, [sa];\n\t}"
-                 : "=r"(v) : "r"(u), "n"(e8_resident(NB)), "l"(packed), "r"(tbase));
+                 : "=r"(v) : "r"(u), "n"(e8_resident(NB, SCALED)), "l"(packed), "r"(tbase));
     return v;
 }
 
@@ -230,7 +238,7 @@ __device__ __forceinline__ CorrUnit corr_begin(const RowsArgs<MAXL>& p, int u, i
     return c;
 }
 // Four batch rows at a time; stores the sums and takes the tile's ticket.  Returns whether it was the last.
-template <int KIND, int NB, int MAXL>
+template <int KIND, int NB, bool SCALED, int MAXL>
 __device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrUnit& c, int lane) {
     float cstar[4] = {0.f, 0.f, 0.f, 0.f};                     // what the main loop adds for a marker (E8: zero)
     if (KIND == EPTQ_E8D4) {
@@ -252,15 +260,16 @@ __device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrU
         float hv = c.h;
         uint4 ov = c.O;
         for (int i = c.lo + sub; i < c.hi;) {
-            float o8[8], xv[4];
+            float o8[8], xv[4], sg = 1.f;
             unpack8(ov, o8);
+            if (SCALED && KIND == EPTQ_E8D4) sg = __half2float(__ldg(L.S + static_cast<size_t>((c.qt * 4 + (lane >> 3)) / L.qb_rows) * L.N + col));
 #pragma unroll
             for (int b = 0; b < 4; ++b)
                 xv[b] = b0 + b < p.B ? hv * __half2float(__ldg(L.x + static_cast<size_t>(b0 + b) * L.N + col)) : 0.f;
 #pragma unroll
             for (int b = 0; b < 4; ++b)
 #pragma unroll
-                for (int k = 0; k < 8; ++k) acc[b][k] = fmaf(o8[k] - cstar[k & 3], xv[b], acc[b][k]);
+                for (int k = 0; k < 8; ++k) acc[b][k] = fmaf(SCALED ? fmaf(-sg, cstar[k & 3], o8[k]) : o8[k] - cstar[k & 3], xv[b], acc[b][k]);
             i += 8;
             if (i < c.hi) {
                 col = __ldg(L.O_col + i);
@@ -288,7 +297,7 @@ __device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrU
     return lane == 0 && last_arrival(p, L, rt);
 }
 
-template <int KIND, int NB, int MAXL>
+template <int KIND, int NB, int MAXL, bool SCALED>
 __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid_constant__ RowsArgs<MAXL> p) {
     constexpr int RING = ring_steps(NB);
     constexpr int BT = NB == 16 ? 2 : 1;                       // accumulator column tiles
@@ -337,12 +346,14 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     Pos pf = cur;
     settle(pf);
     // prefetch pointers of the position: Q row of this lane, x and h columns this thread converts
-    constexpr int XC = NB == 16 ? 4 : NB == 8 ? 2 : 1;         // columns converted per thread
-    const int xrow = ctid / (32 / XC), xcol = (ctid % (32 / XC)) * XC;
+    static_assert(!SCALED || NB == 4, "group scales run in passes of four rows");
+    constexpr int XC = NB == 16 || SCALED ? 4 : NB == 8 ? 2 : 1;         // columns converted per thread
+    const int xtid = SCALED ? lane : ctid;
+    const int xrow = xtid / (32 / XC), xcol = (xtid % (32 / XC)) * XC;
     const bool xlive = xrow < p.B;
-    struct Raw { uint4 q; unsigned x[(XC + 1) / 2], h[(XC + 1) / 2]; };
+    struct Raw { uint4 q; unsigned x[(XC + 1) / 2], h[(XC + 1) / 2], s[SCALED ? 2 : 1]; };
     const int16_t* qp = nullptr;
-    const __half *xp = nullptr, *hp = nullptr;
+    const __half *xp = nullptr, *hp = nullptr, *sp = nullptr;
     auto place = [&]() {
         if (pf.l >= p.n_layers) return;
         const RowsLayer& L = p.L[pf.l];
@@ -350,10 +361,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         qp = L.Q + static_cast<size_t>(row) * L.N + pf.k * 32 + 8 * t;
         xp = L.x + static_cast<size_t>(xlive ? xrow : 0) * L.N + pf.k * 32 + xcol;
         hp = L.h + pf.k * 32 + xcol;
+        if (SCALED) sp = L.S + static_cast<size_t>(min(pf.rt * kTileRows + rg * 8, L.M - 1) / L.qb_rows) * L.N + pf.k * 32 + xcol;
     };
     auto next = [&]() {
         pf.k += kColGroups;
-        if (pf.k < pf.kend) { qp += 32 * kColGroups; xp += 32 * kColGroups; hp += 32 * kColGroups; }
+        if (pf.k < pf.kend) { qp += 32 * kColGroups; xp += 32 * kColGroups; hp += 32 * kColGroups; if (SCALED) sp += 32 * kColGroups; }
         else { settle(pf); place(); }
     };
     auto load_cols = [&](const __half* src, unsigned (&v)[(XC + 1) / 2]) {
@@ -369,13 +381,15 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         ring[i].q = make_uint4(0, 0, 0, 0);
 #pragma unroll
         for (int e = 0; e < (XC + 1) / 2; ++e) { ring[i].x[e] = 0u; ring[i].h[e] = 0u; }
-        if (pf.l < p.n_layers) { ring[i].q = ldg_once(qp); load_cols(hp, ring[i].h); next(); }
+#pragma unroll
+        for (int e = 0; e < (SCALED ? 2 : 1); ++e) ring[i].s[e] = 0u;
+        if (pf.l < p.n_layers) { ring[i].q = ldg_once(qp); load_cols(hp, ring[i].h); if constexpr (SCALED) load_cols(sp, ring[i].s); next(); }
     }
 
     if constexpr (KIND == EPTQ_E8) {
-        const unsigned dst0 = base + e8_table_offset(NB);
+        const unsigned dst0 = base + e8_table_offset(NB, SCALED);
         const char* src0 = reinterpret_cast<const char*>(p.packed);
-        for (unsigned off = tid * 16u; off < e8_resident(NB) * 4u; off += kRowsThreads * 16u)
+        for (unsigned off = tid * 16u; off < e8_resident(NB, SCALED) * 4u; off += kRowsThreads * 16u)
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst0 + off), "l"(src0 + off) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
     } else {
@@ -393,22 +407,22 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         const Pos keep = pf;
-        const int16_t* kq_ = qp; const __half *kx = xp, *kh = hp;
+        const int16_t* kq_ = qp; const __half *kx = xp, *kh = hp, *ks = sp;
         pf = pf0;
         place();
 #pragma unroll
         for (int i = 0; i < RING; ++i)
             if (pf.l < p.n_layers) { if (xlive) load_cols(xp, ring[i].x); next(); }
-        pf = keep; qp = kq_; xp = kx; hp = kh;
+        pf = keep; qp = kq_; xp = kx; hp = kh; sp = ks;
     }
 
     // The first unit's ticket is looked at behind the main loop (its round trip costs nothing there).
     bool corr_last = false;
-    if (unit0 < p.corr_units) corr_last = corr_finish<KIND, NB>(p, corr, lane);
+    if (unit0 < p.corr_units) corr_last = corr_finish<KIND, NB, SCALED>(p, corr, lane);
     const int corr_l = corr.l, corr_rt = corr.qt / kCorrPerTile;
     for (int u = unit0 + unit_step; u < p.corr_units; u += unit_step) {
         const CorrUnit c = corr_begin(p, u, lane);
-        const bool last = corr_finish<KIND, NB>(p, c, lane);
+        const bool last = corr_finish<KIND, NB, SCALED>(p, c, lane);
         if (__any_sync(0xffffffffu, last)) finish_tile<NB>(p, p.L[c.l], c.qt / kCorrPerTile, lane, 32);
         __syncwarp();
     }
@@ -417,12 +431,12 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
 
     const unsigned area = base;                                // fragment buffers / sums over column groups
     unsigned char* const area_p = smem_raw;
-    unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB));
-    const unsigned my_buf = kq * 2 * kBuf;
+    unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB, SCALED));
+    const unsigned my_buf = (SCALED ? warp : kq) * 2 * kBuf;
     const unsigned wr_off = my_buf + ((xcol >> 2) & 1) * kHalf + xrow * 32 + (xcol >> 3) * 8 + (xcol & 3) * 2;
     const unsigned rd_addr = area + my_buf + g * 32 + t * 8;
     const unsigned lane_tab = 8u * (lane & 15) | kRowsTableAddr;
-    const unsigned tbase = base + e8_table_offset(NB);
+    const unsigned tbase = base + e8_table_offset(NB, SCALED);
 
     float acc[BT][4][4];
 #pragma unroll
@@ -504,8 +518,8 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         const unsigned w[4] = {q.x ^ 0x80008000u, q.y ^ 0x80008000u, q.z ^ 0x80008000u, q.w ^ 0x80008000u};
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            e[2 * k] = e8_fetch<NB>(w[k] & 0xFFFFu, tbase, p.packed);
-            e[2 * k + 1] = e8_fetch<NB>(w[k] >> 16, tbase, p.packed);
+            e[2 * k] = e8_fetch<NB, SCALED>(w[k] & 0xFFFFu, tbase, p.packed);
+            e[2 * k + 1] = e8_fetch<NB, SCALED>(w[k] >> 16, tbase, p.packed);
         }
     };
     if constexpr (KIND == EPTQ_E8) lookup(ring[0].q, ent);
@@ -520,7 +534,9 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
             for (int e = 0; e < XC; ++e) {
                 const unsigned short xb = static_cast<unsigned short>(in.x[e >> 1] >> (16 * (e & 1)));
                 const unsigned short hb = static_cast<unsigned short>(in.h[e >> 1] >> (16 * (e & 1)));
-                split_half(__half2float(__ushort_as_half(xb)) * (__half2float(__ushort_as_half(hb)) * sc), hi[e], lo[e]);
+                float hx = __half2float(__ushort_as_half(hb)) * sc;
+                if constexpr (SCALED) hx *= __half2float(__ushort_as_half(static_cast<unsigned short>(in.s[e >> 1] >> (16 * (e & 1)))));
+                split_half(__half2float(__ushort_as_half(xb)) * hx, hi[e], lo[e]);
             }
             unsigned char* w = area_p + wr_off + par * kBuf;
             if constexpr (XC == 4) {
@@ -537,10 +553,12 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         if (pf.l < p.n_layers) {
             in.q = ldg_once(qp);
             load_cols(hp, in.h);
+            if constexpr (SCALED) load_cols(sp, in.s);
             if (xlive) load_cols(xp, in.x);
             next();
         }
-        asm volatile("bar.sync %0, 128;" :: "r"(2 + kq) : "memory");     // the step's fragments are complete
+        if constexpr (SCALED) __syncwarp();
+        else asm volatile("bar.sync %0, 128;" :: "r"(2 + kq) : "memory");     // the step's fragments are complete
         const unsigned rd = rd_addr + par * kBuf;
         par ^= 1;
         unsigned ahead[8];
@@ -616,14 +634,14 @@ bool plan_rows(const EptqLayer* layers, int n, int B, int n_sms, RowsPlan& plan)
     return true;
 }
 
-template <int KIND, int NB, int MAXL>
+template <int KIND, int NB, bool SCALED = false, int MAXL>
 int launch_kernel(const RowsArgs<MAXL>& a, int n_sms, cudaStream_t stream) {
     constexpr int smem = KIND == EPTQ_E8 ? kRowsSmemE8 : kRowsSmemD4;
     static std::atomic<bool> attr_done[64];       // setting the attribute twice is harmless; the flag itself must not race
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return EPTQ_ERR_LAUNCH;
     if (!attr_done[dev]) {
-        if (cudaFuncSetAttribute(gemv_rows_kernel<KIND, NB, MAXL>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+        if (cudaFuncSetAttribute(gemv_rows_kernel<KIND, NB, MAXL, SCALED>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
             return EPTQ_ERR_LAUNCH;
         attr_done[dev] = true;
     }
@@ -637,7 +655,7 @@ int launch_kernel(const RowsArgs<MAXL>& a, int n_sms, cudaStream_t stream) {
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    const cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_rows_kernel<KIND, NB, MAXL>, a);
+    const cudaError_t err = cudaLaunchKernelEx(&cfg, gemv_rows_kernel<KIND, NB, MAXL, SCALED>, a);
     count_launch(EPTQ_KERNEL_GEMV_GROUP);
     return err == cudaSuccess ? EPTQ_OK : EPTQ_ERR_LAUNCH;
 }
@@ -673,9 +691,11 @@ int launch_sized(const RowsPlan& plan, const EptqLayer* layers, int n, const uin
         R.ns = L.N / 32;
         R.row_tiles = (L.M + kTileRows - 1) / kTileRows;
         R.step0 = step0; R.tile0 = tile0; R.corr0 = corr0;
+        R.S = reinterpret_cast<const __half*>(L.S_group);
+        R.qb_rows = L.S_group != nullptr ? L.qb_size / 8 : 0;
         R.corr_tile = L.n_masked != 0 ? kCorrPerTile : 0;      // -1 (count unknown): the row pointers carry it
         int e = 0;
-        std::frexp(L.h_absmax, &e);            // h_absmax = m * 2^e, m in [0.5, 1)  =>  2^-e <= 1/h_absmax
+        std::frexp(std::fabs(L.h_absmax), &e);            // h_absmax = m * 2^e, m in [0.5, 1)  =>  2^-e <= 1/h_absmax
         R.x_scale = std::ldexp(1.0f, -e);
         R.x_inv_scale = std::ldexp(1.0f, e) * (e8 ? L.table_packed_scale : 1.0f);
         step0 += R.row_tiles * R.ns;
@@ -683,6 +703,8 @@ int launch_sized(const RowsPlan& plan, const EptqLayer* layers, int n, const uin
         corr0 += R.row_tiles * R.corr_tile;
     }
     a.corr_units = corr0;
+    if constexpr (MAXL == kRowsFewLayers)
+        if (layers[0].S_group != nullptr) return e8 ? launch_kernel<EPTQ_E8, 4, true>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 4, true>(a, plan.G, stream);
     switch (rows_of(B)) {
         case 4: return e8 ? launch_kernel<EPTQ_E8, 4>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 4>(a, plan.G, stream);
         case 8: return e8 ? launch_kernel<EPTQ_E8, 8>(a, plan.G, stream) : launch_kernel<EPTQ_E8D4, 8>(a, plan.G, stream);
@@ -704,6 +726,28 @@ int launch_gemv_rows(const EptqLayer* layers, int n, const uint16_t* const* xs, 
     if (!plan_rows(layers, n, B, n_sms, plan)) return EPTQ_ERR_UNSUPPORTED;
     return n <= kRowsFewLayers ? launch_sized<kRowsFewLayers>(plan, layers, n, xs, ys, B, workspace, stream)
                                : launch_sized<kRowsMaxLayers>(plan, layers, n, xs, ys, B, workspace, stream);
+}
+
+// One layer with group scales that are constant over 64 outputs; -h_absmax = max|h| * max|S_group| bounds x*h*S.
+bool rows_scaled_supported(const EptqLayer& L, int B) {
+    return L.S_group != nullptr && L.qb_size > 0 && (L.qb_size % 64) == 0 && L.h_absmax < 0.f && std::isfinite(L.h_absmax) && B >= 1 && B <= kGemmMinBatch &&
+           (L.N % 32) == 0 && aligned16(L.Q) && aligned16(L.h) && aligned16(L.g) && aligned16(L.S_group) &&
+           (L.bias == nullptr || aligned16(L.bias)) && (L.n_masked == 0 || aligned16(L.O_vals)) &&
+           (L.quantizer == EPTQ_E8 ? L.table_packed != nullptr && aligned16(L.table_packed) && L.table_packed_scale > 0.f
+                                   : L.table16 != nullptr && aligned16(L.table16));
+}
+
+// Passes of four rows, the scratch of rows_workspace_bytes(&L, 1, 4, n_sms).
+int launch_gemv_rows_scaled(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B, int n_sms, void* workspace, cudaStream_t stream) {
+    RowsPlan plan;
+    if (!plan_rows(&L, 1, 4, n_sms, plan)) return EPTQ_ERR_UNSUPPORTED;
+    for (int b = 0; b < B; b += 4) {
+        const uint16_t* xs[1] = {x + static_cast<size_t>(b) * L.N};
+        uint16_t* ys[1] = {y + static_cast<size_t>(b) * 8 * L.M};
+        const int st = launch_sized<kRowsFewLayers>(plan, &L, 1, xs, ys, B - b < 4 ? B - b : 4, workspace, stream);
+        if (st != EPTQ_OK) return st;
+    }
+    return EPTQ_OK;
 }
 
 }  // namespace eptq

@@ -279,6 +279,8 @@ def _make_desc(quantizer_type: str, Q, table32, table16, g, h, O_vals, O_col, O_
     d.bias, d.S_group = _ptr(bias), _ptr(S_group)
     d.table8, d.table8_scale = None, 0.0
     d.h_absmax = h_absmax(h) if Q.is_cuda else 0.0
+    if S_group is not None:
+        d.h_absmax *= -h_absmax(S_group) if Q.is_cuda else 0.0       # the bound of h * S_group, marked by its sign
     d.table_packed, d.table_packed_scale = None, 0.0
     d.crit_ptr = d.crit_pos = d.crit_O = None
     if crit is not None:

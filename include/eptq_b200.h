@@ -105,7 +105,8 @@ typedef struct EptqLayer {
     const uint16_t* S_group;
     const uint8_t* table8;
     float table8_scale;
-    float h_absmax;           /* max |h|, or 0 if not known (then the persistent GEMV is not used) */
+    float h_absmax;           /* max |h|, or 0 if not known (then the persistent GEMV is not used); for a layer with
+                                 group scales -max|h| * max|S_group| opens the multi-row GEMV, any other value does not */
     const uint32_t* table_packed; /* E8 only, optional: 65536 packed entries, see below */
     float table_packed_scale;
     int32_t reserved;
@@ -212,8 +213,8 @@ int eptq_linear_forward(const EptqLayer* layer, const uint16_t* x, uint16_t* y,
  * Requirements: layers of one codebook (E8-D4 sharing one table16, or E8 sharing
  * one table_packed), no group scales, N % 32 == 0, h_absmax set, B <= 16;
  * otherwise EPTQ_ERR_UNSUPPORTED (call eptq_linear_forward per layer instead).
- * One launch covers two batch rows; larger B is run as ceil(B/2) launches over
- * the same weights.  `xs` / `ys` are host arrays of device pointers.  Scratch as for eptq_linear_forward, size from
+ * Above two rows one launch covers all of them if the scratch has the size eptq_group_workspace_bytes
+ * states; with 1 MiB only, B rows run as ceil(B/2) launches over the same weights.  `xs` / `ys` are host arrays of device pointers.  Scratch as for eptq_linear_forward, size from
  * eptq_group_workspace_bytes.
  */
 size_t eptq_group_workspace_bytes(const EptqLayer* layers, int n_layers, int B);

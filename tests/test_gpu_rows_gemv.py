@@ -73,3 +73,24 @@ def test_small_scratch_takes_passes_of_two_rows(kind):
                                        torch.cuda.current_stream().cuda_stream)
     assert st == 0
     check(kind, qds, [x, x], ys)
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("out,inn,qb,batch", [(2048, 4096, 128, 1), (1536, 5504, 512, 3), (4160, 2080, 64, 5), (2048, 4128, 2048, 16)])
+def test_group_scales_match_oracle(kind, out, inn, qb, batch):
+    """Group scales in passes of four rows; scales that span a factor of about a thousand."""
+    from eptq_b200.kernels import h_absmax
+    qd = make_layer(out, inn, seed=out + qb, outlier_frac=0.01, bias=(batch % 2 == 1), qb_size=qb)
+    gen = torch.Generator().manual_seed(qb)
+    qd.S_group = torch.exp(1.2 * torch.randn(qd.S_group.shape, generator=gen)).to(torch.float16)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV)
+    x = make_activations(batch, inn, seed=qb + batch)
+    before = _lib.load().eptq_kernel_launch_count(1)
+    y = lin(x.to(DEV))
+    torch.cuda.synchronize()
+    assert _lib.load().eptq_kernel_launch_count(1) - before == (batch + 3) // 4       # the multi-row kernel took it
+    assert lin.descriptor().h_absmax == pytest.approx(-h_absmax(lin.h) * h_absmax(lin.S_group))
+    W16 = oracle.dequantize_layer(util.qld_arrays(qd), TABLES[kind])
+    ref = oracle.linear_reference(x.numpy(), W16, None if qd.bias is None else qd.bias.numpy())
+    for b in range(batch):
+        assert util.max_rel_err(y[b].float().cpu().numpy(), ref[b]) <= util.REL_TOL
