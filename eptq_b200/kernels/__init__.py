@@ -213,19 +213,24 @@ def e8_packed(table: torch.Tensor) -> Optional[Tuple[torch.Tensor, float]]:
 _absmax_cache: Dict[tuple, float] = {}
 
 
-def h_absmax(h: torch.Tensor) -> float:
-    """max |h| of a column-scale vector, computed once per tensor (one device sync) and cached.
-    The persistent GEMV derives its activation scale from it."""
+def h_absmax(h: torch.Tensor, scales: Optional[torch.Tensor] = None) -> float:
+    """max |h| of a column-scale vector, times max |scales| if group scales are given; computed once per tensor (one
+    device sync) and cached.  The persistent GEMV derives its activation scale from it."""
     key = (h.data_ptr(), h.device, h.numel(), h._version)
+    if scales is not None:
+        key += (scales.data_ptr(), scales.numel(), scales._version)
     v = _absmax_cache.get(key)
     if v is None:
-        v = float(h.abs().max().item()) if h.numel() else 0.0
+        top = h.abs().max().float() if h.numel() else torch.zeros(())
+        if scales is not None and scales.numel() and h.numel():
+            top = top * scales.abs().max().float()
+        v = float(top.item())
         if len(_absmax_cache) > 4096:
             for k in [k for k in _cache_sources if k[0] == "absmax"]:
                 del _cache_sources[k]
             _absmax_cache.clear()
         _absmax_cache[key] = v
-        _cache_sources[("absmax",) + key] = h
+        _cache_sources[("absmax",) + key] = (h, scales)
     return v
 
 
@@ -278,9 +283,8 @@ def _make_desc(quantizer_type: str, Q, table32, table16, g, h, O_vals, O_col, O_
     d.O_vals, d.O_col, d.O_row_ptr = _ptr(O_vals), _ptr(O_col), O_row_ptr.data_ptr()
     d.bias, d.S_group = _ptr(bias), _ptr(S_group)
     d.table8, d.table8_scale = None, 0.0
-    d.h_absmax = h_absmax(h) if Q.is_cuda else 0.0
-    if S_group is not None:
-        d.h_absmax *= -h_absmax(S_group) if Q.is_cuda else 0.0       # the bound of h * S_group, marked by its sign
+    # with group scales: the bound of h * S_group, marked by its sign
+    d.h_absmax = 0.0 if not Q.is_cuda else h_absmax(h) if S_group is None else -h_absmax(h, S_group)
     d.table_packed, d.table_packed_scale = None, 0.0
     d.crit_ptr = d.crit_pos = d.crit_O = None
     if crit is not None:

@@ -22,7 +22,7 @@ import torch
 import torch.nn as nn
 
 from .. import _lib
-from . import _make_desc, critical_lists, d4_table8, h_absmax, linear_forward
+from . import _make_desc, critical_lists, d4_table8, linear_forward
 
 MARKER = 32767     # int16 value that marks a critical block (index 65535 - 32768)
 
@@ -94,9 +94,6 @@ class EPTQLinear(nn.Module):
                                   unit=t8[1] if t8 is not None else None, code_max=float(codebook.abs().max()))
         for name, t in zip(("crit_ptr", "crit_pos", "crit_O"), crit):
             self.register_buffer(name, t, persistent=False)
-
-        if self.S_group is not None and self.S_group.is_cuda:
-            h_absmax(self.S_group)                   # read back once here, not in the first call
 
         # Shared between layers, therefore plain attributes, not buffers.
         self._codebook = codebook
