@@ -678,7 +678,7 @@ def run_gpu_arm(args):
                                                  "prefill_s": st["prefill_s"],
                                                  "config": f"llama2-70b architecture, random init, 80 layers, E8 r=1.6, 1024-token "
                                                            f"prompt + 32 greedy tokens, batch 1, tp{world}"}
-                # the same weights at batch 8 (GEMV passes of two rows; reductions of 8 x 8192 values go through NCCL)
+                # the same weights at batch 8 (one GEMV pass for all rows; reductions of 8 x 8192 values go through NCCL)
                 from eptq_b200.engine import LlamaDecodeEngine
                 layers70 = eng.layers
                 head70 = (eng.embed, eng.final_norm, eng.lm_head, eng.inv_freq, eng.eps, eng.head_dim, eng.n_heads, eng.n_kv_heads)

@@ -1,9 +1,9 @@
 // Prefill GEMM on an already reconstructed fp16 weight (tcgen05 + TMEM + TMA), sm_100a.
 //
-// For long prefills the weight is reconstructed ONCE by dequant_kernel (bit-exact fp16, the reference's
+// For long prefills the weight is reconstructed ONCE by dequant.cu (bit-exact fp16, the reference's
 // dequantize_layer) into scratch, and this kernel multiplies: y (T, out) = x (T, in) * W16 (out, in)^T (+ bias),
 // fp32 accumulation in tensor memory.  The fused kernel (gemm_tcgen05_ws.cu) reconstructs every weight tile once
-// per 512 tokens at ~35 instructions per index, which is what holds it at 40 % of the tensor peak; here both
+// per 512 tokens, which is what holds it at 40 % of the tensor peak; here both
 // operands arrive by TMA and no thread touches them.
 //
 //   tile      256 tokens x 256 outputs per block: two accumulators of 128 lanes x 256 TMEM columns.
