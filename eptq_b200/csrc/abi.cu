@@ -196,7 +196,7 @@ size_t eptq_workspace_bytes(int M, int N, int B) {
         const size_t grp = group_workspace_bytes(&shape, 1, B, 0);
         if (grp > bytes) bytes = grp;
     }
-    if (B >= kDenseMinTokens && (N % 8) == 0 && kPartialOffset + dense_weight_bytes(M, N) > bytes)
+    if (B >= kDenseShapeTokens && (N % 8) == 0 && kPartialOffset + dense_weight_bytes(M, N) > bytes)
         bytes = kPartialOffset + dense_weight_bytes(M, N);
     return (bytes + 255) & ~static_cast<size_t>(255);
 }

@@ -39,7 +39,13 @@ constexpr size_t kCounterBytes = 4096;
 constexpr size_t kPartialOffset = 1u << 20;
 constexpr int kMaxCounters = static_cast<int>(kCounterBytes / sizeof(unsigned));
 constexpr int kGemmMinBatch = 16;           // batches above this run on the tensor-core GEMM
-constexpr int kDenseMinTokens = 1024;       // from here on the weight is reconstructed once into scratch and a dense GEMM follows
+// From kDenseMinTokens on the weight is reconstructed once into scratch and a dense GEMM follows, if the scratch has room
+// (eptq_layer_workspace_bytes asks for it).  Up to 512 tokens one token tile reads each weight once anyway, and there K
+// ranges fill the SMs where the dense GEMM does not (4096 x 11008 E8-D4 at 300 tokens: 72 against 85 us).  At 700 tokens,
+// tile by tile against once: 4096 x 4096 E8-D4 68.5 / 46.4 us, 11008 x 4096 160 / 80 us, 4096 x 11008 130 / 101 us,
+// 1024 x 4096 53.7 / 30.1 us; E8 79.4 / 52.0, 195 / 100, 155 / 121, 57.6 / 32.8 us.
+constexpr int kDenseMinTokens = 513;
+constexpr int kDenseShapeTokens = 1024;     // from here on eptq_workspace_bytes, which knows the shape only, counts that room
 // The last counter word is the GEMM's status word (EPTQ_ERR_TIMEOUT if a bounded wait ran out), so
 // GEMV plans may use at most kMaxCounters - 1 counters.
 

@@ -150,9 +150,9 @@ int eptq_prepare_d4_table8(const float* table, uint8_t* out, float* scale);
  */
 size_t eptq_workspace_bytes(int M, int N, int B);
 /* The same from the layer itself: for prefill-sized B when the tensor-core GEMM takes the layer, the first
- * 1 MiB only (16 < B < 1024) or 1 MiB + 16*M*N bytes (B >= 1024: the fp16 weight is reconstructed once into the
- * scratch and a dense GEMM follows; with a smaller scratch the call still works and reconstructs tile by tile);
- * eptq_workspace_bytes(M, N, B) otherwise. */
+ * 1 MiB plus the partial sums of its K ranges (16 < B <= 512) or 1 MiB + 16*M*N bytes (B > 512: the fp16 weight is
+ * reconstructed once into the scratch and a dense GEMM follows); with a smaller scratch the call still works, with
+ * one K range and reconstructing tile by tile; eptq_workspace_bytes(M, N, B), or more for group scales, otherwise. */
 size_t eptq_layer_workspace_bytes(const EptqLayer* layer, int B);
 
 /*
