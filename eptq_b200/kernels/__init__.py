@@ -16,9 +16,11 @@ Inputs must be CUDA tensors; a CPU tensor raises -- there is no CPU path.
 from __future__ import annotations
 
 import ctypes as C
+import weakref
 from typing import Dict, Optional, Tuple
 
 import torch
+from torch.utils.weak import WeakTensorKeyDictionary
 
 from .. import _lib
 
@@ -213,24 +215,37 @@ def e8_packed(table: torch.Tensor) -> Optional[Tuple[torch.Tensor, float]]:
 _absmax_cache: Dict[tuple, float] = {}
 
 
-def h_absmax(h: torch.Tensor, scales: Optional[torch.Tensor] = None) -> float:
-    """max |h| of a column-scale vector, times max |scales| if group scales are given; computed once per tensor (one
-    device sync) and cached.  The persistent GEMV derives its activation scale from it."""
+def h_absmax(h: torch.Tensor) -> float:
+    """max |h| of a column-scale vector, computed once per tensor (one device sync) and cached.
+    The persistent GEMV derives its activation scale from it."""
     key = (h.data_ptr(), h.device, h.numel(), h._version)
-    if scales is not None:
-        key += (scales.data_ptr(), scales.numel(), scales._version)
     v = _absmax_cache.get(key)
     if v is None:
-        top = h.abs().max().float() if h.numel() else torch.zeros(())
-        if scales is not None and scales.numel() and h.numel():
-            top = top * scales.abs().max().float()
-        v = float(top.item())
+        v = float(h.abs().max().item()) if h.numel() else 0.0
         if len(_absmax_cache) > 4096:
             for k in [k for k in _cache_sources if k[0] == "absmax"]:
                 del _cache_sources[k]
             _absmax_cache.clear()
         _absmax_cache[key] = v
-        _cache_sources[("absmax",) + key] = (h, scales)
+        _cache_sources[("absmax",) + key] = h
+    return v
+
+
+# group scales -> (column scales, their versions and addresses, max |h| * max |S_group|); holds neither tensor
+_scaled_bounds = WeakTensorKeyDictionary()
+
+
+def scaled_absmax(h: torch.Tensor, scales: torch.Tensor) -> float:
+    """max |h| * max |scales|, one device sync for both the first time a layer asks."""
+    tag = (h._version, h.data_ptr(), scales._version, scales.data_ptr())
+    hit = _scaled_bounds.get(scales)
+    if hit is not None and hit[0]() is h and hit[1] == tag:
+        return hit[2]
+    v = 0.0
+    if h.numel() and scales.numel():
+        v = float((torch.linalg.vector_norm(h, float("inf"), dtype=torch.float32)
+                   * torch.linalg.vector_norm(scales, float("inf"), dtype=torch.float32)).item())
+    _scaled_bounds[scales] = (weakref.ref(h), tag, v)
     return v
 
 
@@ -284,7 +299,7 @@ def _make_desc(quantizer_type: str, Q, table32, table16, g, h, O_vals, O_col, O_
     d.bias, d.S_group = _ptr(bias), _ptr(S_group)
     d.table8, d.table8_scale = None, 0.0
     # with group scales: the bound of h * S_group, marked by its sign
-    d.h_absmax = 0.0 if not Q.is_cuda else h_absmax(h) if S_group is None else -h_absmax(h, S_group)
+    d.h_absmax = 0.0 if not Q.is_cuda else h_absmax(h) if S_group is None else -scaled_absmax(h, S_group)
     d.table_packed, d.table_packed_scale = None, 0.0
     d.crit_ptr = d.crit_pos = d.crit_O = None
     if crit is not None:
