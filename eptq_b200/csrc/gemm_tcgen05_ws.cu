@@ -154,7 +154,7 @@ gemm_tcgen05_ws_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(16) float4 tab_s[KIND == EPTQ_E8D4 ? 512 : 1];
     __shared__ __align__(8) unsigned long long bar_full[kMaxStages], bar_empty[kMaxStages], bar_qfull[kQStages], bar_qempty[kQStages], bar_acc;
-    __shared__ unsigned tmem_base_slot, last_slot;
+    __shared__ unsigned tmem_base_slot, last_slot, read_sink[kProducerWarps];
 
     constexpr int kStages = ws_stages(KIND, TM, NT);
     constexpr int kStageBytes = ws_stage_bytes(TM, NT);
@@ -312,8 +312,14 @@ gemm_tcgen05_ws_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
                 if (s_shared) in.s = *reinterpret_cast<const unsigned*>(src + kQBytes + kChunkK * 2);
                 else if (srow != nullptr) in.s = __ldg(reinterpret_cast<const unsigned*>(srow + n0));
             }
-            __syncwarp();
-            if (lane == 0) mbar_arrive(smem_u32(&bar_qempty[s]));
+            // The slot is free for the next TMA write once every lane's values are in registers.  An arrive alone does not
+            // wait for that: shared-memory reads still under way saw the slot's next chunk.  So the arrive follows a store
+            // that needs all of them.
+            const unsigned read = __reduce_xor_sync(0xffffffffu, in.q ^ in.h ^ in.s);
+            if (lane == 0) {
+                *static_cast<volatile unsigned*>(&read_sink[qrow]) = read;
+                mbar_arrive(smem_u32(&bar_qempty[s]));
+            }
             return true;
         };
         int next_marker = b_valid ? first_marker(L, bm, c_begin * kChunkK) : 0;

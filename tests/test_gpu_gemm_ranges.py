@@ -4,6 +4,7 @@ import pytest
 import torch
 
 import oracle
+from eptq_b200 import _lib
 from eptq_b200.kernels.linear import EPTQLinear
 from eptq_b200.synthetic import make_activations, make_layer
 from tests import util
@@ -34,3 +35,31 @@ def test_ranges_match_oracle(kind, out, inn, tokens, qb, frac):
     assert torch.equal(lin(xd), y)                       # ranges are added in a fixed order, the scratch is left clean
     W = lin.dequantize()
     assert np.array_equal(W.cpu().numpy().view(np.uint16), np.asarray(W16).view(np.uint16))     # bit-exact
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("tokens", [100, 200, 400])
+@pytest.mark.parametrize("one_range", [False, True])
+def test_every_column_meets_its_own_weight(kind, tokens, one_range):
+    """One-hot rows read the weights the GEMM multiplied by: a column of W16 each, exactly.  Blocks with many chunks, so
+    that the index ring is refilled while the slowest warp still reads it; cold and warm L2."""
+    import ctypes as C
+    out = inn = 4096
+    lin = EPTQLinear.from_quantized_data(make_layer(out, inn, seed=3, device=DEV), torch.from_numpy(TABLES[kind]).to(DEV), kind)
+    W = lin.dequantize()
+    d = lin.descriptor()
+    lib = _lib.load()
+    need = 1 << 20 if one_range else lib.eptq_layer_workspace_bytes(C.byref(d), tokens)
+    ws = torch.zeros(need, dtype=torch.uint8, device=DEV)
+    flush = torch.empty(1 << 28, dtype=torch.uint8, device=DEV)
+    rows = torch.arange(tokens, device=DEV)
+    for rep in range(16):
+        cols = (rows * inn // tokens + 5 * rep) % inn
+        x = torch.zeros((tokens, inn), dtype=torch.float16, device=DEV)
+        x[rows, cols] = 1
+        if rep % 2 == 0:
+            flush.zero_()
+        y = torch.empty((tokens, out), dtype=torch.float16, device=DEV)
+        st = lib.eptq_linear_forward(C.byref(d), x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(), ws.numel(),
+                                     torch.cuda.current_stream().cuda_stream)
+        assert st == 0 and torch.equal(y, W[:, cols].T)
