@@ -4,14 +4,16 @@
 // What bounds a small layer's call is this path, not the kernel: written in Python over ctypes it took 23 us per
 // call (module attribute lookups of five buffers, two scratch-size calls, descriptor structures rebuilt for every
 // grouped call) beside kernels of 3 to 10 us.  A LayerHandle keeps the EptqLayer descriptor of a module's device
-// buffers; a call checks by identity that the module still holds those buffers and then only touches the ATen
-// allocator and the library.
+// buffers; a call checks that the module still holds the same buffers, unchanged where the descriptor holds a value
+// computed from them, and then only touches the ATen allocator and the library.
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <ATen/ATen.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
+#include <cstring>
 #include <map>
 #include <utility>
 #include <vector>
@@ -21,16 +23,29 @@
 namespace {
 
 constexpr const char* kCapsule = "eptq_b200.LayerHandle";
-constexpr const char* kBufferNames[3] = {"Q", "g", "h"};
+// Every buffer the descriptor points into.  It also holds the maxima of h and S_group, so those may not change in place.
+constexpr const char* kBufferNames[] = {"Q", "g", "h", "O_vals", "O_col", "O_row_ptr", "bias", "S_group", "crit_ptr", "crit_pos", "crit_O"};
+constexpr int kBuffers = sizeof(kBufferNames) / sizeof(kBufferNames[0]);
+constexpr int kOptionalFrom = 6;                                     // bias and what follows may be None
+constexpr bool kHoldsValue[kBuffers] = {false, false, true, false, false, false, false, true, false, false, false};
+constexpr int kTables = 2;                                           // the fp16 and the fp32 codebook
 constexpr size_t kMinScratch = 1u << 20;
 constexpr int kSmallRows = 16;
+
+// A tensor as it was when the descriptor was made, or None.
+struct Held {
+    PyObject* obj = nullptr;            // owned
+    const void* ptr = nullptr;
+    int64_t numel = 0;
+    int64_t version = 0;
+};
 
 struct LayerHandle {
     EptqLayer d;
     PyObject* keep;                     // tensors (and host tables) the descriptor points into
     PyObject* buffers;                  // the module's _buffers dict
-    PyObject* held[3];                  // Q, g, h as they were when the descriptor was made (owned)
-    const void* held_ptr[3];
+    Held held[kBuffers];
+    Held tables[kTables];
     int64_t in_features, out_features;
     size_t scratch[kSmallRows + 1];     // eptq_layer_workspace_bytes for small batches, 0 = not asked yet
 };
@@ -40,19 +55,47 @@ void free_handle(PyObject* capsule) {
     if (h == nullptr) { PyErr_Clear(); return; }
     Py_XDECREF(h->keep);
     Py_XDECREF(h->buffers);
-    for (PyObject* o : h->held) Py_XDECREF(o);
+    for (const Held& t : h->held) Py_XDECREF(t.obj);
+    for (const Held& t : h->tables) Py_XDECREF(t.obj);
     delete h;
 }
 
 LayerHandle* handle_of(PyObject* o) { return static_cast<LayerHandle*>(PyCapsule_GetPointer(o, kCapsule)); }
 
-// The module still holds the buffers the descriptor was made from (replacing or moving one makes a new tensor or
-// a new address).
+int64_t version_of(const at::Tensor& t) { return t.is_inference() ? 0 : static_cast<int64_t>(t._version()); }
+
+void hold(Held& h, PyObject* o) {
+    h.obj = Py_NewRef(o);
+    if (o == Py_None) return;
+    const at::Tensor& t = THPVariable_Unpack(o);
+    h.ptr = t.const_data_ptr();
+    h.numel = t.numel();
+    h.version = version_of(t);
+}
+
+bool unchanged(const Held& h, bool value) {
+    if (h.obj == Py_None) return true;
+    const at::Tensor& t = THPVariable_Unpack(h.obj);
+    return t.const_data_ptr() == h.ptr && t.numel() == h.numel && (!value || version_of(t) == h.version);
+}
+
+PyObject* const* buffer_keys() {
+    static PyObject** keys = [] {
+        auto** k = new PyObject*[kBuffers];
+        for (int i = 0; i < kBuffers; ++i) k[i] = PyUnicode_InternFromString(kBufferNames[i]);
+        return k;
+    }();
+    return keys;
+}
+
+// The descriptor still describes the module: the same buffers (replacing or moving one makes a new tensor or a new
+// address), and unchanged values where it holds one: max|h|, max|S_group|, the codebooks' lattice scale and packed form.
 bool is_current(const LayerHandle* h) {
-    for (int i = 0; i < 3; ++i) {
-        PyObject* now = PyDict_GetItemString(h->buffers, kBufferNames[i]);        // borrowed
-        if (now != h->held[i] || THPVariable_Unpack(now).const_data_ptr() != h->held_ptr[i]) return false;
-    }
+    PyObject* const* keys = buffer_keys();
+    for (int i = 0; i < kBuffers; ++i)
+        if (PyDict_GetItem(h->buffers, keys[i]) != h->held[i].obj || !unchanged(h->held[i], kHoldsValue[i])) return false;
+    for (const Held& t : h->tables)
+        if (!unchanged(t, true)) return false;
     return true;
 }
 
@@ -116,35 +159,49 @@ PyObject* wrap(at::Tensor y, at::ScalarType dtype) {
     return THPVariable_Wrap(dtype == at::kHalf ? std::move(y) : y.to(dtype));
 }
 
-// make_handle(descriptor bytes, keep, buffers dict, in_features, out_features)
+// make_handle(descriptor bytes, keep, buffers dict, (fp16 codebook, fp32 codebook or None), in_features, out_features)
 PyObject* make_handle(PyObject*, PyObject* const* a, Py_ssize_t n) {
-    if (n != 5 || !PyBytes_Check(a[0]) || PyBytes_GET_SIZE(a[0]) != static_cast<Py_ssize_t>(sizeof(EptqLayer)) || !PyDict_Check(a[2])) {
-        PyErr_SetString(PyExc_TypeError, "make_handle(descriptor, keep, buffers, in_features, out_features)");
+    HANDLE_TH_ERRORS
+    if (n != 6 || !PyBytes_Check(a[0]) || PyBytes_GET_SIZE(a[0]) != static_cast<Py_ssize_t>(sizeof(EptqLayer)) ||
+        !PyDict_Check(a[2]) || !PyTuple_Check(a[3]) || PyTuple_GET_SIZE(a[3]) != kTables) {
+        PyErr_SetString(PyExc_TypeError, "make_handle(descriptor, keep, buffers, codebooks, in_features, out_features)");
         return nullptr;
     }
-    const long long in = PyLong_AsLongLong(a[3]), out = PyLong_AsLongLong(a[4]);
+    const long long in = PyLong_AsLongLong(a[4]), out = PyLong_AsLongLong(a[5]);
     if (PyErr_Occurred()) return nullptr;
-    PyObject* held[3];
-    for (int i = 0; i < 3; ++i) {
-        held[i] = PyDict_GetItemString(a[2], kBufferNames[i]);
-        if (held[i] == nullptr || !THPVariable_Check(held[i])) {
-            PyErr_SetString(PyExc_TypeError, "make_handle: buffers Q, g and h must be tensors");
+    PyObject* held[kBuffers];
+    for (int i = 0; i < kBuffers; ++i) {
+        held[i] = PyDict_GetItem(a[2], buffer_keys()[i]);
+        if (held[i] == nullptr || !(THPVariable_Check(held[i]) || (i >= kOptionalFrom && held[i] == Py_None))) {
+            PyErr_Format(PyExc_TypeError, "make_handle: buffer %s must be a tensor%s", kBufferNames[i], i >= kOptionalFrom ? " or None" : "");
+            return nullptr;
+        }
+    }
+    for (int i = 0; i < kTables; ++i) {
+        PyObject* o = PyTuple_GET_ITEM(a[3], i);
+        if (!THPVariable_Check(o) && o != Py_None) {
+            PyErr_SetString(PyExc_TypeError, "make_handle: codebooks must be tensors or None");
             return nullptr;
         }
     }
     auto* h = new LayerHandle();
-    std::memcpy(&h->d, PyBytes_AS_STRING(a[0]), sizeof(EptqLayer));
     h->keep = Py_NewRef(a[1]);
     h->buffers = Py_NewRef(a[2]);
-    for (int i = 0; i < 3; ++i) {
-        h->held[i] = Py_NewRef(held[i]);
-        h->held_ptr[i] = THPVariable_Unpack(held[i]).const_data_ptr();
+    PyObject* c = PyCapsule_New(h, kCapsule, free_handle);               // owns h, also if what follows throws
+    if (c == nullptr) {
+        Py_DECREF(h->keep);
+        Py_DECREF(h->buffers);
+        delete h;
+        return nullptr;
     }
+    THPObjectPtr owner(c);
+    std::memcpy(&h->d, PyBytes_AS_STRING(a[0]), sizeof(EptqLayer));
+    for (int i = 0; i < kBuffers; ++i) hold(h->held[i], held[i]);
+    for (int i = 0; i < kTables; ++i) hold(h->tables[i], PyTuple_GET_ITEM(a[3], i));
     h->in_features = in;
     h->out_features = out;
-    PyObject* c = PyCapsule_New(h, kCapsule, free_handle);
-    if (c == nullptr) delete h;
-    return c;
+    return owner.release();
+    END_HANDLE_TH_ERRORS
 }
 
 // forward(handle, x) -> y, or None if the module's buffers are no longer the descriptor's
@@ -259,7 +316,7 @@ PyObject* dequantize(PyObject*, PyObject* const* a, Py_ssize_t n) {
         return nullptr;
     }
     if (!is_current(h)) Py_RETURN_NONE;
-    const at::Tensor& q = THPVariable_Unpack(h->held[0]);
+    const at::Tensor& q = THPVariable_Unpack(h->held[0].obj);
     if (!q.is_cuda()) {
         PyErr_SetString(PyExc_RuntimeError, "eptq_b200: `Q` must be a CUDA tensor (no CPU path exists)");
         return nullptr;

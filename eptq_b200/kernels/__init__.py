@@ -283,7 +283,7 @@ def critical_lists(O_vals: torch.Tensor, O_col: torch.Tensor, O_row_ptr: torch.T
 
 
 def _make_desc(quantizer_type: str, Q, table32, table16, g, h, O_vals, O_col, O_row_ptr, bias, S_group,
-               qb_size: int, crit=None) -> _lib.EptqLayer:
+               qb_size: int, crit=None, bounds: bool = True) -> _lib.EptqLayer:
     d = _lib.EptqLayer()
     d.quantizer = _lib.QUANTIZER_ID[quantizer_type]
     d.M, d.N = Q.shape
@@ -299,7 +299,7 @@ def _make_desc(quantizer_type: str, Q, table32, table16, g, h, O_vals, O_col, O_
     d.bias, d.S_group = _ptr(bias), _ptr(S_group)
     d.table8, d.table8_scale = None, 0.0
     # with group scales: the bound of h * S_group, marked by its sign
-    d.h_absmax = 0.0 if not Q.is_cuda else h_absmax(h) if S_group is None else -scaled_absmax(h, S_group)
+    d.h_absmax = 0.0 if not (Q.is_cuda and bounds) else h_absmax(h) if S_group is None else -scaled_absmax(h, S_group)
     d.table_packed, d.table_packed_scale = None, 0.0
     d.crit_ptr = d.crit_pos = d.crit_O = None
     if crit is not None:

@@ -47,6 +47,10 @@ def _shared_table(codebook: torch.Tensor, dtype: torch.dtype, quantizer_type: st
     return tab
 
 
+# Plain attributes the descriptor is made from; the native host path watches the buffers itself.
+_DESCRIBED = frozenset(("in_features", "out_features", "quantizer_type", "qb_size", "_codebook", "_codebook32"))
+
+
 class EPTQLinear(nn.Module):
     """Quantized linear layer computing ``y = x W^T + bias`` straight from
     ``Q`` (int16 (out/8, in)), the codebook, ``g``, ``h`` and the critical blocks."""
@@ -99,6 +103,16 @@ class EPTQLinear(nn.Module):
         self._codebook = codebook
         self._codebook32 = codebook32
         self._handle = None          # descriptor of the device buffers for the native host path
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name in _DESCRIBED:
+            self.__dict__["_handle"] = None
+
+    def _replicate_for_data_parallel(self):
+        replica = super()._replicate_for_data_parallel()
+        replica._handle = None                     # it describes the original's buffers
+        return replica
 
     def _apply(self, fn, *args, **kwargs):
         super()._apply(fn, *args, **kwargs)
@@ -177,13 +191,19 @@ class EPTQLinear(nn.Module):
 
     def _new_handle(self):
         """Native handle of the current buffers; the host path says (by returning None) when they have been
-        replaced or moved since, and a new one is made."""
+        replaced, moved or changed since, and a new one is made.  The maxima of h and S_group are read back from
+        the GPU then, which a stream capture does not allow: a handle renewed inside one serves that call only and
+        leaves them out (kernels that need none)."""
         if not self.Q.is_cuda:
             raise RuntimeError("EPTQLinear runs on CUDA tensors only (there is no CPU path)")
-        d = self.descriptor()
-        keep = (d, tuple(self._buffers.values()), self._codebook, self._codebook32)
-        self._handle = _lib.host().make_handle(bytes(d), keep, self._buffers, self.in_features, self.out_features)
-        return self._handle
+        passing = self._handle is not None and torch.cuda.is_current_stream_capturing()
+        d = self._describe(bounds=not passing)
+        tables = (self._codebook, self._codebook32)
+        keep = (d, tuple(self._buffers.values()), tables)
+        handle = _lib.host().make_handle(bytes(d), keep, self._buffers, tables, self.in_features, self.out_features)
+        if not passing:
+            self._handle = handle
+        return handle
 
     def __getstate__(self):
         state = super().__getstate__() if hasattr(super(), "__getstate__") else self.__dict__
@@ -199,9 +219,12 @@ class EPTQLinear(nn.Module):
 
     def descriptor(self):
         """The C-ABI description (struct EptqLayer) of this layer's device buffers."""
+        return self._describe()
+
+    def _describe(self, bounds: bool = True):
         crit = (self.crit_ptr, self.crit_pos, self.crit_O) if self.crit_ptr is not None else None
         return _make_desc(self.quantizer_type, self.Q, self._codebook32, self._codebook, self.g, self.h,
-                          self.O_vals, self.O_col, self.O_row_ptr, self.bias, self.S_group, self.qb_size, crit)
+                          self.O_vals, self.O_col, self.O_row_ptr, self.bias, self.S_group, self.qb_size, crit, bounds)
 
     def extra_repr(self) -> str:
         return (f"in={self.in_features}, out={self.out_features}, quantizer={self.quantizer_type}, "

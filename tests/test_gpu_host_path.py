@@ -1,0 +1,85 @@
+"""The native host path of module calls: it follows the module it was made for."""
+import pytest
+import torch
+
+import oracle
+from eptq_b200.kernels.linear import EPTQLinear, forward_group
+from eptq_b200.synthetic import make_activations, make_layer
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+_tables: dict = {}
+
+
+def table(kind):
+    """One codebook tensor: layers of a group share it."""
+    if kind not in _tables:
+        _tables[kind] = torch.from_numpy(oracle.d4_table(1.75) if kind == "e8_d4" else oracle.e8_table(1.6)).to(DEV)
+    return _tables[kind]
+
+
+def layer(kind, out=1024, inn=2048, seed=1, **kw):
+    qd = make_layer(out, inn, seed=seed, device=DEV, outlier_frac=0.01, **kw)
+    return EPTQLinear.from_quantized_data(qd, table(kind), kind)
+
+
+def fresh(lin):
+    """A new module over the present buffers."""
+    return EPTQLinear(lin.Q, lin._codebook, lin.g, lin.h, lin.O_vals, lin.O_col, lin.O_row_ptr, lin.bias, lin.quantizer_type,
+                      S_group=lin.S_group, codebook32=lin._codebook32)
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("tokens", [1, 3])
+def test_calls_follow_changed_buffers(kind, tokens):
+    lin, other = layer(kind, bias=True), layer(kind, seed=2)
+    x = make_activations(tokens, 2048, seed=9, device=DEV)
+    changes = [
+        lambda: setattr(lin, "bias", lin.bias * -3),
+        lambda: setattr(lin, "g", lin.g * 2),
+        lambda: setattr(lin, "O_vals", lin.O_vals * 4) or setattr(lin, "crit_O", fresh(lin).crit_O),
+        lambda: lin.h.mul_(1000),                       # in place: x * h * 2^-e would leave fp16 with the old bound
+        lambda: lin.h.div_(4000),
+        lambda: setattr(lin, "bias", None),
+    ]
+    lin.g.mul_(2.0 ** -8)
+    for change in [lambda: None, *changes]:
+        change()
+        ref = fresh(lin)
+        assert torch.allclose(lin(x).float(), ref(x).float(), rtol=2e-3, atol=2e-3 * float(ref(x).float().abs().max()))
+        a, b = forward_group([lin, other], [x, x])
+        ra, rb = forward_group([ref, other], [x, x])
+        assert torch.isfinite(a).all() and torch.allclose(a.float(), ra.float(), rtol=2e-3, atol=2e-3 * float(ra.float().abs().max()))
+        assert torch.equal(lin.dequantize(), ref.dequantize())
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_group_scales_follow_changed_buffers(kind):
+    lin = layer(kind, out=4096, inn=2048, qb_size=128)
+    x = make_activations(1, 2048, seed=9, device=DEV)
+    lin.g.mul_(2.0 ** -12)
+    for change in (lambda: None, lambda: lin.S_group.mul_(4096), lambda: setattr(lin, "S_group", lin.S_group / 512)):
+        change()
+        ref = fresh(lin)
+        y, r = lin(x).float(), ref(x).float()
+        assert torch.isfinite(y).all() and torch.allclose(y, r, rtol=2e-3, atol=2e-3 * float(r.abs().max()))
+        assert torch.equal(lin.dequantize(), ref.dequantize())
+
+
+def test_changed_scales_then_capture():
+    """A capture cannot read the new maxima back; the call is recorded with kernels that need none."""
+    lin = layer("e8_d4")
+    x = make_activations(1, 2048, seed=9, device=DEV)
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        lin(x)
+        lin.h.mul_(0.5)
+        side.synchronize()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=side):
+            y = lin(x)
+        graph.replay()
+        side.synchronize()
+    ref = fresh(lin)(x).float()
+    assert torch.allclose(y.float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))
+    assert torch.allclose(lin(x).float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))

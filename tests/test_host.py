@@ -125,3 +125,62 @@ def test_critical_lists_group_blocks_by_unit_and_check_their_range(built_library
     assert none == (None, None, None)
     ok = critical_lists(lin.O_vals, lin.O_col, lin.O_row_ptr, N, unit=0.1, code_max=2.0)
     assert ok[0] is not None and CRIT_ROW_LIMIT > 0
+
+
+def _handle(lin):
+    """A native handle of a CPU module: its launches refuse CPU tensors, its checks run."""
+    from eptq_b200 import _lib
+    d = lin.descriptor()
+    tables = (lin._codebook, lin._codebook32)
+    keep = (d, tuple(lin._buffers.values()), tables)
+    return _lib.host().make_handle(bytes(d), keep, lin._buffers, tables, lin.in_features, lin.out_features)
+
+
+def _described(lin, handle):
+    """Whether the host path takes the handle for the module's present state (None: make a new one)."""
+    from eptq_b200 import _lib
+    try:
+        return _lib.host().dequantize(handle) is not None
+    except RuntimeError as e:
+        assert "CUDA" in str(e)
+        return True
+
+
+@pytest.mark.parametrize("name", ["Q", "g", "h", "O_vals", "O_col", "O_row_ptr", "bias", "S_group", "crit_ptr", "crit_pos", "crit_O"])
+def test_handle_notices_a_replaced_buffer(built_library, name):
+    qd = make_layer(64, 32, seed=3, outlier_frac=0.1, bias=True, qb_size=None if name.startswith("crit") else 32)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(oracle.d4_table(1.75)), "e8_d4")
+    handle = _handle(lin)
+    assert _described(lin, handle)
+    setattr(lin, name, getattr(lin, name).clone())
+    assert not _described(lin, handle) and _described(lin, _handle(lin))
+    handle = _handle(lin)
+    getattr(lin, name).data = getattr(lin, name).clone()          # same object, other memory
+    assert not _described(lin, handle)
+    if name in ("bias", "S_group"):
+        handle = _handle(lin)
+        setattr(lin, name, None)
+        assert not _described(lin, handle)
+
+
+@pytest.mark.parametrize("name", ["h", "S_group", "_codebook", "_codebook32"])
+def test_handle_notices_values_changed_in_place(built_library, name):
+    """The descriptor holds numbers computed from these."""
+    qd = make_layer(64, 32, seed=3, outlier_frac=0.1, qb_size=32)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(oracle.d4_table(1.75)).clone(), "e8_d4")
+    handle = _handle(lin)
+    getattr(lin, name).mul_(2)
+    assert not _described(lin, handle) and _described(lin, _handle(lin))
+
+
+def test_handle_is_dropped_with_what_it_was_made_from(built_library):
+    import copy
+    lin = EPTQLinear.from_quantized_data(make_layer(64, 32, seed=3), torch.from_numpy(oracle.d4_table(1.75)), "e8_d4")
+    for name in ("_codebook", "_codebook32", "qb_size", "quantizer_type", "in_features", "out_features"):
+        lin._handle = _handle(lin)
+        setattr(lin, name, getattr(lin, name))
+        assert lin._handle is None
+    lin._handle = _handle(lin)
+    assert lin._replicate_for_data_parallel()._handle is None
+    assert copy.deepcopy(lin)._handle is None and copy.copy(lin)._handle is None
+    assert lin._handle is not None
