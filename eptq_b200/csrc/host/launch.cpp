@@ -101,7 +101,8 @@ bool is_current(const LayerHandle* h) {
 
 // One zero-filled scratch tensor per (device, stream), grown on demand; only touched with the GIL held.  A CUDA graph
 // keeps the addresses it was captured with, so a tensor handed out during a capture is kept when a larger one
-// replaces it.
+// replaces it.  A caller owns the tensor it gets until its launches are enqueued: the GIL is released for them, and
+// another thread on the same stream may replace the map's tensor meanwhile.
 struct Scratch { at::Tensor t; bool captured = false; };
 std::map<std::pair<int, int64_t>, Scratch>& scratch_map() {
     static auto* m = new std::map<std::pair<int, int64_t>, Scratch>();            // never destroyed: no CUDA calls at exit
@@ -113,7 +114,7 @@ std::vector<std::pair<int, at::Tensor>>& kept_scratch() {
     return *v;
 }
 
-const at::Tensor& scratch_for(int device, const c10::cuda::CUDAStream& stream, size_t bytes) {
+at::Tensor scratch_for(int device, const c10::cuda::CUDAStream& stream, size_t bytes) {
     Scratch& s = scratch_map()[{device, static_cast<int64_t>(reinterpret_cast<intptr_t>(stream.stream()))}];
     if (!s.t.defined() || static_cast<size_t>(s.t.numel()) < bytes) {
         if (s.captured) kept_scratch().emplace_back(device, std::move(s.t));
@@ -226,7 +227,7 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
         need = eptq_layer_workspace_bytes(&h->d, static_cast<int>(B));
         if (B <= kSmallRows) h->scratch[B] = need;
     }
-    const at::Tensor& ws = scratch_for(x.device().index(), stream, need);
+    const at::Tensor ws = scratch_for(x.device().index(), stream, need);
     void* const ws_ptr = ws.data_ptr();
     const size_t ws_bytes = static_cast<size_t>(ws.numel());
     const auto* xp = static_cast<const uint16_t*>(rows.const_data_ptr());
@@ -291,7 +292,7 @@ PyObject* forward_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         return nullptr;
     }
     const auto stream = c10::cuda::getCurrentCUDAStream(device.index());
-    const at::Tensor& ws = scratch_for(device.index(), stream, need);
+    const at::Tensor ws = scratch_for(device.index(), stream, need);
     void* const ws_ptr = ws.data_ptr();
     const size_t ws_bytes = static_cast<size_t>(ws.numel());
     int st;

@@ -83,3 +83,55 @@ def test_changed_scales_then_capture():
     ref = fresh(lin)(x).float()
     assert torch.allclose(y.float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))
     assert torch.allclose(lin(x).float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))
+
+
+def in_threads(jobs):
+    """Run the jobs at the same time, switching between them as often as the interpreter can; errors surface."""
+    import sys
+    import threading
+    errors = []
+    start = threading.Barrier(len(jobs))
+
+    def body(job):
+        try:
+            start.wait()
+            job()
+        except BaseException as e:                      # noqa: BLE001 - reported below
+            errors.append(e)
+
+    interval = sys.getswitchinterval()
+    sys.setswitchinterval(1e-6)
+    try:
+        threads = [threading.Thread(target=body, args=(job,)) for job in jobs]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+    finally:
+        sys.setswitchinterval(interval)
+    if errors:
+        raise errors[0]
+
+
+def test_scratch_outgrown_by_another_thread():
+    """One thread's calls keep the scratch they were given while another's replace it with larger ones."""
+    lin = layer("e8_d4", out=2048, inn=2048)
+    small, big = make_activations(40, 2048, seed=4, device=DEV), make_activations(500, 2048, seed=5, device=DEV)
+    want_small, want_big = lin(small), {t: lin(big[:t].contiguous()) for t in range(100, 501, 50)}
+    for _ in range(5):
+        side = torch.cuda.Stream()                      # a stream without scratch
+        side.wait_stream(torch.cuda.current_stream())
+
+        def steady():
+            with torch.cuda.stream(side):
+                for _ in range(200):
+                    assert torch.equal(lin(small), want_small)
+
+        def growing():
+            with torch.cuda.stream(side):
+                for t, want in want_big.items():
+                    torch.full((1 << 20,), 255, dtype=torch.uint8, device=DEV)          # takes freed memory
+                    assert torch.equal(lin(big[:t].contiguous()), want)
+
+        in_threads([steady, growing])
+    torch.cuda.synchronize()
