@@ -73,8 +73,26 @@ size_t dense_weight_bytes(int M, int N) {
     return (static_cast<size_t>(8) * M * N * sizeof(uint16_t) + 255) & ~static_cast<size_t>(255);
 }
 
+// A call of several launches keeps its own data in the scratch between them (the reconstructed weight a dense GEMM reads),
+// so another thread's call on the same scratch may not be enqueued in between.  Held while a call is enqueued, by the
+// scratch it uses; two scratches that share a lock only wait for each other's enqueue.
+class EnqueueLock {
+public:
+    explicit EnqueueLock(const void* workspace) {
+        if (workspace != nullptr) lock_ = std::unique_lock<std::mutex>(mutexes()[(reinterpret_cast<uintptr_t>(workspace) >> 12) % kStripes]);
+    }
+private:
+    static constexpr int kStripes = 61;
+    static std::mutex* mutexes() {
+        static auto* m = new std::mutex[kStripes];       // never destroyed: calls may come from other threads at exit
+        return m;
+    }
+    std::unique_lock<std::mutex> lock_;
+};
+
 int forward_checked(const EptqLayer& L, const uint16_t* x, uint16_t* y, int B,
                     void* workspace, size_t workspace_bytes, void* stream) {
+    const EnqueueLock lock(workspace);
     int st = check_layer_common(&L);
     if (st != EPTQ_OK) return st;
     if (x == nullptr || y == nullptr || L.table16 == nullptr) return EPTQ_ERR_NULL;
@@ -234,6 +252,7 @@ int eptq_linear_forward_group_fused(const EptqLayer* layers, int n_layers, const
         if (!aligned16(xs[i])) return EPTQ_ERR_ALIGN;
     }
     if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return EPTQ_ERR_ALIGN;
+    const EnqueueLock lock(workspace);
     if (stream_gemv_supported(layers, n_layers, B))
         return launch_gemv_stream(layers, n_layers, fusions, nullptr, xs, ys, B, workspace, workspace_bytes,
                                   static_cast<cudaStream_t>(stream));
@@ -255,6 +274,7 @@ int eptq_linear_forward_chain(const EptqLayer* layers, int n_layers, const EptqF
     }
     if (workspace != nullptr && (reinterpret_cast<uintptr_t>(workspace) & 255u) != 0) return EPTQ_ERR_ALIGN;
     if (!stream_gemv_supported(layers, n_layers, B)) return EPTQ_ERR_UNSUPPORTED;
+    const EnqueueLock lock(workspace);
     return launch_gemv_stream(layers, n_layers, fusions, phases, xs, ys, B, workspace, workspace_bytes,
                               static_cast<cudaStream_t>(stream));
 }

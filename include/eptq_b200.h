@@ -146,7 +146,10 @@ int eptq_prepare_d4_table8(const float* table, uint8_t* out, float* scale);
  * for every call that is ordered on one stream, for layers of any shape (take
  * the maximum of the sizes): the first 1 MiB holds counters and accumulators
  * that every kernel returns to zero, the rest is overwritten before it is
- * read.  Calls that may overlap on the GPU need separate scratch.
+ * read.  Calls that may overlap on the GPU need separate scratch.  Several threads may
+ * call with one scratch and one stream: a call's launches are enqueued without another
+ * call's between them.  (A graph that holds such a call is not: do not replay it on the
+ * stream while another thread calls with the scratch it was captured with.)
  */
 size_t eptq_workspace_bytes(int M, int N, int B);
 /* The same from the layer itself: for prefill-sized B when the tensor-core GEMM takes the layer, the first

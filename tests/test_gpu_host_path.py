@@ -135,3 +135,21 @@ def test_scratch_outgrown_by_another_thread():
 
         in_threads([steady, growing])
     torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("tokens", [600, 1100])
+def test_two_threads_reconstruct_into_one_scratch(tokens):
+    """Above 512 tokens a call reconstructs its weight into the stream's scratch and multiplies from there."""
+    lins = [layer(kind, out=1024, inn=1024, seed=n) for n, kind in enumerate(("e8_d4", "e8_d4", "e8_lattice"))]
+    x = make_activations(tokens, 1024, seed=4, device=DEV)
+    decode = layer("e8_d4", out=2048, inn=2048, seed=7)                     # one launch, partial sums in the same place
+    xd = make_activations(8, 2048, seed=5, device=DEV)
+    want, want_d = [lin(x) for lin in lins], decode(xd)
+
+    def repeat(lin, x, want):
+        def job():
+            got = [lin(x) for _ in range(150)]
+            assert all(torch.equal(y, want) for y in got)
+        return job
+
+    in_threads([repeat(lin, x, w) for lin, w in zip(lins, want)] + [repeat(decode, xd, want_d)])
