@@ -55,6 +55,8 @@ class EPTQLinear(nn.Module):
     """Quantized linear layer computing ``y = x W^T + bias`` straight from
     ``Q`` (int16 (out/8, in)), the codebook, ``g``, ``h`` and the critical blocks."""
 
+    _handle = None          # modules pickled before the handle existed have none in their state
+
     def __init__(
         self,
         Q: torch.Tensor,

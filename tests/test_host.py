@@ -184,3 +184,15 @@ def test_handle_is_dropped_with_what_it_was_made_from(built_library):
     assert lin._replicate_for_data_parallel()._handle is None
     assert copy.deepcopy(lin)._handle is None and copy.copy(lin)._handle is None
     assert lin._handle is not None
+
+
+def test_module_pickled_without_a_handle_still_calls(built_library):
+    lin = EPTQLinear.from_quantized_data(make_layer(64, 32, seed=3), torch.from_numpy(oracle.d4_table(1.75)), "e8_d4")
+    state = dict(lin.__getstate__())
+    del state["_handle"]
+    state["_desc"] = None                              # what such a pickle held in its place
+    back = EPTQLinear.__new__(EPTQLinear)
+    back.__setstate__(state)
+    for call in (lambda: back(torch.zeros(1, 32, dtype=torch.float16)), back.dequantize):
+        with pytest.raises(RuntimeError, match="CUDA"):          # reaches the host path, which refuses CPU tensors
+            call()
