@@ -134,13 +134,15 @@ bool fail(int status, const char* what) {
     return false;
 }
 
-// x as contiguous fp16 rows of in_features; false with a Python error set if it cannot be.
-bool as_rows(const LayerHandle* h, const at::Tensor& x, at::Tensor& rows, int64_t& n_rows) {
+// x as contiguous fp16 rows of in_features; false with a Python error set if it cannot be.  With `reshape` its own
+// dimensions do not matter (the output takes another input's), its values only have to fill whole rows.
+bool as_rows(const LayerHandle* h, const at::Tensor& x, at::Tensor& rows, int64_t& n_rows, bool reshape = false) {
     if (!x.is_cuda()) {
         PyErr_SetString(PyExc_RuntimeError, "EPTQLinear runs on CUDA tensors only (there is no CPU path)");
         return false;
     }
-    if (x.dim() < 1 || x.size(-1) != h->in_features) {
+    const bool whole = reshape && h->in_features > 0 && x.numel() % h->in_features == 0;
+    if (!whole && (x.dim() < 1 || x.size(-1) != h->in_features)) {
         PyErr_Format(PyExc_RuntimeError, "EPTQLinear: the last dimension of the input must be %lld", (long long)h->in_features);
         return false;
     }
@@ -242,8 +244,8 @@ PyObject* forward(PyObject*, PyObject* const* a, Py_ssize_t n) {
     END_HANDLE_TH_ERRORS
 }
 
-// forward_group(handles, xs) -> list of outputs, or None if some module's buffers have changed.  All inputs have
-// the leading shape of the first.
+// forward_group(handles, xs) -> list of outputs, or None if some module's buffers have changed.  All outputs have
+// the leading shape of the first input.
 PyObject* forward_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
     HANDLE_TH_ERRORS
     if (n_args != 2 || !PyList_Check(a[0]) || !PyList_Check(a[1]) || PyList_GET_SIZE(a[0]) != PyList_GET_SIZE(a[1]) ||
@@ -270,7 +272,7 @@ PyObject* forward_group(PyObject*, PyObject* const* a, Py_ssize_t n_args) {
         if (!is_current(h)) Py_RETURN_NONE;
         const at::Tensor& x = THPVariable_Unpack(xo);
         int64_t b = 0;
-        if (!as_rows(h, x, rows[i], b)) return nullptr;
+        if (!as_rows(h, x, rows[i], b, i > 0)) return nullptr;
         if (i == 0) {
             B = b;
             device = x.device();

@@ -153,3 +153,17 @@ def test_two_threads_reconstruct_into_one_scratch(tokens):
         return job
 
     in_threads([repeat(lin, x, w) for lin, w in zip(lins, want)] + [repeat(decode, xd, want_d)])
+
+
+def test_group_inputs_of_other_shapes():
+    """Inputs after the first may have any shape with as many values, attention heads not yet joined for instance."""
+    a, b = layer("e8_d4"), layer("e8_d4", seed=2)
+    x, z = make_activations(3, 2048, seed=9, device=DEV), make_activations(3, 2048, seed=8, device=DEV)
+    ya, yb = forward_group([a, b], [x, z])
+    for other in (z.view(3, 16, 128), z.view(-1), z.view(1, 3, 2048), z.view(3, 1, 2048).float()):
+        oa, ob = forward_group([a, b], [x, other])
+        assert torch.equal(oa, ya) and torch.equal(ob, yb.to(other.dtype)) and ob.shape == yb.shape
+    with pytest.raises(RuntimeError):
+        forward_group([a, b], [x, z.view(-1)[:-1]])
+    with pytest.raises(RuntimeError):
+        forward_group([a, b], [x, z[:2]])
