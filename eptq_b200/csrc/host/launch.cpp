@@ -102,7 +102,9 @@ bool is_current(const LayerHandle* h) {
 // One zero-filled scratch tensor per (device, stream), grown on demand; only touched with the GIL held.  A CUDA graph
 // keeps the addresses it was captured with, so a tensor handed out during a capture is kept when a larger one
 // replaces it.  A caller owns the tensor it gets until its launches are enqueued: the GIL is released for them, and
-// another thread on the same stream may replace the map's tensor meanwhile.
+// another thread on the same stream may replace the map's tensor meanwhile.  Whether a graph is gone is not known here,
+// so a kept tensor stays; its successor has at least twice its size, which bounds all that a stream keeps by the size of
+// the scratch it has.
 struct Scratch { at::Tensor t; bool captured = false; };
 std::map<std::pair<int, int64_t>, Scratch>& scratch_map() {
     static auto* m = new std::map<std::pair<int, int64_t>, Scratch>();            // never destroyed: no CUDA calls at exit
@@ -117,8 +119,11 @@ std::vector<std::pair<int, at::Tensor>>& kept_scratch() {
 at::Tensor scratch_for(int device, const c10::cuda::CUDAStream& stream, size_t bytes) {
     Scratch& s = scratch_map()[{device, static_cast<int64_t>(reinterpret_cast<intptr_t>(stream.stream()))}];
     if (!s.t.defined() || static_cast<size_t>(s.t.numel()) < bytes) {
-        if (s.captured) kept_scratch().emplace_back(device, std::move(s.t));
-        const int64_t n = static_cast<int64_t>(bytes > kMinScratch ? bytes : kMinScratch);
+        int64_t n = static_cast<int64_t>(bytes > kMinScratch ? bytes : kMinScratch);
+        if (s.captured) {
+            if (n < 2 * s.t.numel()) n = 2 * s.t.numel();
+            kept_scratch().emplace_back(device, std::move(s.t));
+        }
         s.t = at::zeros({n}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, static_cast<c10::DeviceIndex>(device)));
         s.captured = false;
     }

@@ -167,3 +167,31 @@ def test_group_inputs_of_other_shapes():
         forward_group([a, b], [x, z.view(-1)[:-1]])
     with pytest.raises(RuntimeError):
         forward_group([a, b], [x, z[:2]])
+
+
+def test_scratch_kept_for_graphs_is_bounded():
+    """Scratch a graph was captured with outlives its replacement; what is kept stays below what is in use."""
+    from eptq_b200 import _lib
+    host = _lib.host()
+    index = torch.cuda.current_device()
+    before = {t.data_ptr() for t in host.scratch_of_device(index)}
+    lin = layer("e8_d4", out=2048, inn=1024)
+    side = torch.cuda.Stream()
+    graphs = []
+    with torch.cuda.stream(side):
+        for t in range(600, 1000, 50):                  # each asks for a little more scratch than the one before
+            big = layer("e8_d4", out=2 * t // 16 * 16, inn=1024, seed=t)
+            x = make_activations(t, 1024, seed=t, device=DEV)
+            want = big(x)
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=side):
+                y = big(x)
+            graphs.append((graph, big, x, y, want))
+        for graph, _, _, y, want in graphs:
+            y.zero_()
+            graph.replay()
+            assert torch.equal(y, want)
+        lin(make_activations(1, 1024, seed=1, device=DEV))
+        current = host.scratch(index, 1)
+    sizes = [t.numel() for t in host.scratch_of_device(index) if t.data_ptr() not in before and t.data_ptr() != current.data_ptr()]
+    assert sizes and sum(sizes) <= current.numel()
