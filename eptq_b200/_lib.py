@@ -10,7 +10,15 @@ from pathlib import Path
 from typing import Optional
 
 LIB_PATH = Path(__file__).resolve().parent / "lib" / "libeptq_b200.so"
-HOST_PATH = LIB_PATH.with_name("_eptq_host.so")
+
+
+def host_path() -> Path:
+    """The host extension for this interpreter and this torch: it links against both."""
+    import sys
+
+    import torch
+    return LIB_PATH.with_name(f"_eptq_host.{sys.implementation.cache_tag}.torch{torch.__version__}.so")
+
 
 EPTQ_E8, EPTQ_E8D4 = 0, 1
 QUANTIZER_ID = {"e8_lattice": EPTQ_E8, "e8_d4": EPTQ_E8D4}
@@ -109,12 +117,12 @@ def host():
         import importlib.machinery
         import importlib.util
 
-        import torch  # noqa: F401  (the extension resolves its symbols against torch's libraries)
         load()
-        if not HOST_PATH.exists():
-            raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m eptq_b200.build`")
-        loader = importlib.machinery.ExtensionFileLoader("_eptq_host", str(HOST_PATH))
-        spec = importlib.util.spec_from_file_location("_eptq_host", str(HOST_PATH), loader=loader)
+        path = host_path()                   # imports torch, whose libraries the extension's symbols are found in
+        if not path.exists():
+            raise RuntimeError(f"{path} is missing: build it with `python -m eptq_b200.build`")
+        loader = importlib.machinery.ExtensionFileLoader("_eptq_host", str(path))
+        spec = importlib.util.spec_from_file_location("_eptq_host", str(path), loader=loader)
         mod = importlib.util.module_from_spec(spec)
         loader.exec_module(mod)
         _host = mod

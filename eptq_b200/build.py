@@ -1,5 +1,5 @@
 """Builds ``lib/libeptq_b200.so`` from ``csrc/*.cu`` with nvcc for sm_100a and the host extension
-``lib/_eptq_host.so`` from ``csrc/host/*.cpp`` with g++.
+``lib/_eptq_host.*.so`` from ``csrc/host/*.cpp`` with g++, named after the interpreter and the torch it is built for.
 
 Run as ``python -m eptq_b200.build``.  nvcc cross-compiles without a GPU.  The
 library has no dependency on torch or Python; it exports the C ABI declared in
@@ -17,7 +17,6 @@ PKG = Path(__file__).resolve().parent
 CSRC = PKG / "csrc"
 LIB_DIR = PKG / "lib"
 LIB_PATH = LIB_DIR / "libeptq_b200.so"
-HOST_PATH = LIB_DIR / "_eptq_host.so"
 HEADER = PKG.parent / "include" / "eptq_b200.h"
 
 NVCC_FLAGS = [
@@ -75,8 +74,9 @@ def build_library(force: bool = False, verbose: bool = False) -> Path:
 
 
 def _build_host(force: bool, verbose: bool) -> None:
-    srcs = sorted((CSRC / "host").glob("*.cpp"))
-    if not force and not _newer(srcs + [HEADER], HOST_PATH):
+    from ._lib import host_path
+    srcs, path = sorted((CSRC / "host").glob("*.cpp")), host_path()
+    if not force and not _newer(srcs + [HEADER], path):
         return
     import sysconfig
 
@@ -87,7 +87,7 @@ def _build_host(force: bool, verbose: bool) -> None:
     cmd = [shutil.which("g++") or "g++", "-O2", "-std=c++17", "-shared", "-fPIC",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
            *[f"-isystem{p}" for p in (*include_paths(), sysconfig.get_paths()["include"], cuda_inc)],
-           *map(str, srcs), "-o", str(HOST_PATH), f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
+           *map(str, srcs), "-o", str(path), f"-L{torch_lib}", "-lc10", "-lc10_cuda", "-ltorch", "-ltorch_cpu",
            "-ltorch_python", f"-L{LIB_DIR}", "-l:libeptq_b200.so", "-Wl,-rpath,$ORIGIN"]
     _run(cmd, "g++", verbose)
 

@@ -196,3 +196,13 @@ def test_module_pickled_without_a_handle_still_calls(built_library):
     for call in (lambda: back(torch.zeros(1, 32, dtype=torch.float16)), back.dequantize):
         with pytest.raises(RuntimeError, match="CUDA"):          # reaches the host path, which refuses CPU tensors
             call()
+
+
+def test_host_extension_is_the_one_for_this_torch(built_library, monkeypatch):
+    """A build for another interpreter or torch is reported, not loaded."""
+    from eptq_b200 import _lib
+    assert _lib.host_path().exists()
+    monkeypatch.setattr(_lib, "_host", None)
+    monkeypatch.setattr(torch, "__version__", "0.0.0")
+    with pytest.raises(RuntimeError, match="build"):
+        _lib.host()
