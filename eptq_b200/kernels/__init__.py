@@ -123,10 +123,22 @@ def _(Q, codes, g, h, x, O_vals, O_col, O_row_ptr, bias):
     return x.new_empty(x.shape[0], Q.shape[0] * 8, dtype=torch.float16)
 
 
-_table8_cache: Dict[tuple, Optional[Tuple[torch.Tensor, float]]] = {}
-# Derived values are cached by the address of their source tensor; the cache keeps that tensor alive, so that the
-# allocator cannot hand the address to another tensor while an entry is valid.  clear_derived_caches() drops all.
-_cache_sources: Dict[tuple, torch.Tensor] = {}
+# Derived values are cached by the address of their source tensor; an entry keeps that tensor alive, so that the
+# allocator cannot hand the address to another tensor while it is valid.  The entry used longest ago goes first: the
+# tables of a model that is being built or called stay, and its layers keep sharing them.
+_table8_cache: Dict[tuple, tuple] = {}
+_packed_cache: Dict[tuple, tuple] = {}
+_absmax_cache: Dict[tuple, tuple] = {}
+
+
+def _cached(cache: Dict[tuple, tuple], key: tuple, source: torch.Tensor, make, limit: int = 64):
+    entry = cache.pop(key, None)
+    if entry is None:
+        entry = (make(), source)
+    cache[key] = entry
+    while len(cache) > limit:
+        cache.pop(next(iter(cache)), None)
+    return entry[0]
 
 
 def clear_derived_caches() -> None:
@@ -134,8 +146,6 @@ def clear_derived_caches() -> None:
     _table8_cache.clear()
     _packed_cache.clear()
     _absmax_cache.clear()
-    _cache_sources.clear()
-
 
 
 def d4_table8(table: torch.Tensor):
@@ -143,26 +153,18 @@ def d4_table8(table: torch.Tensor):
     scale * integer lattice coordinates, or None if the table is not such a multiple
     (a radially warped codebook).  Prepared on the host once per table tensor; the
     library copies it into the kernel parameters at each launch."""
-    key = (table.data_ptr(), table.device, table.dtype, table._version)
-    if key in _table8_cache:
-        return _table8_cache[key]
-    import numpy as np
-    host = np.ascontiguousarray(table.detach().float().cpu().numpy().reshape(-1))
-    res = None
-    if host.size == 2048:
+    def make():
+        import numpy as np
+        host = np.ascontiguousarray(table.detach().float().cpu().numpy().reshape(-1))
+        if host.size != 2048:
+            return None
         out = np.zeros(2048, dtype=np.uint8)
         scale = C.c_float(0.0)
         st = _lib.load().eptq_prepare_d4_table8(host.ctypes.data, out.ctypes.data, C.addressof(scale))
-        if st == 0:
-            res = (out.view(np.int8), float(scale.value))
-    if len(_table8_cache) > 64:
-        _table8_cache.clear()
-    _table8_cache[key] = res
-    _cache_sources[("t8",) + key] = table          # the keyed tensor stays alive: its address cannot be reused
-    return res
+        return (out.view(np.int8), float(scale.value)) if st == 0 else None
+    return _cached(_table8_cache, (table.data_ptr(), table.device, table.dtype, table._version), table, make)
 
 
-_packed_cache: Dict[tuple, Optional[Tuple[torch.Tensor, float]]] = {}
 _E8_FIELD = (0, 4, 1, 5, 2, 6, 3, 7)      # 4-bit field index of dimension d; field f sits at bit 2 + 4 f
 
 
@@ -204,31 +206,14 @@ def unpack_e8_table(word: torch.Tensor, scale: float) -> torch.Tensor:
 def e8_packed(table: torch.Tensor) -> Optional[Tuple[torch.Tensor, float]]:
     """pack_e8_table cached per table tensor (one host sync the first time)."""
     key = (table.data_ptr(), table.device, table.dtype, tuple(table.shape), table._version)
-    if key not in _packed_cache:
-        if len(_packed_cache) > 64:
-            _packed_cache.clear()
-        _packed_cache[key] = pack_e8_table(table)
-        _cache_sources[("packed",) + key] = table
-    return _packed_cache[key]
-
-
-_absmax_cache: Dict[tuple, float] = {}
+    return _cached(_packed_cache, key, table, lambda: pack_e8_table(table))
 
 
 def h_absmax(h: torch.Tensor) -> float:
     """max |h| of a column-scale vector, computed once per tensor (one device sync) and cached.
     The persistent GEMV derives its activation scale from it."""
     key = (h.data_ptr(), h.device, h.numel(), h._version)
-    v = _absmax_cache.get(key)
-    if v is None:
-        v = float(h.abs().max().item()) if h.numel() else 0.0
-        if len(_absmax_cache) > 4096:
-            for k in [k for k in _cache_sources if k[0] == "absmax"]:
-                del _cache_sources[k]
-            _absmax_cache.clear()
-        _absmax_cache[key] = v
-        _cache_sources[("absmax",) + key] = h
-    return v
+    return _cached(_absmax_cache, key, h, lambda: float(h.abs().max().item()) if h.numel() else 0.0, limit=4096)
 
 
 # group scales -> (column scales, their versions and addresses, max |h| * max |S_group|); holds neither tensor

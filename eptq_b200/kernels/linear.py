@@ -22,7 +22,7 @@ import torch
 import torch.nn as nn
 
 from .. import _lib
-from . import _make_desc, critical_lists, d4_table8, linear_forward
+from . import _cached, _make_desc, critical_lists, d4_table8, linear_forward
 
 MARKER = 32767     # int16 value that marks a critical block (index 65535 - 32768)
 
@@ -33,18 +33,11 @@ def _shared_table(codebook: torch.Tensor, dtype: torch.dtype, quantizer_type: st
     """One converted copy per (source tensor, dtype): layers of a model share it."""
     key = (codebook.data_ptr(), codebook.device, tuple(codebook.shape), codebook.dtype, dtype,
            codebook._version, quantizer_type)
-    hit = _table_cache.get(key)
-    if hit is not None:
-        return hit
-    tab = codebook.detach().to(dtype=dtype)
-    tab = tab.reshape(512, 4) if quantizer_type == "e8_d4" else tab
-    tab = tab.contiguous()
-    if len(_table_cache) > 64:
-        from . import clear_derived_caches
-        _table_cache.clear()
-        clear_derived_caches()                 # their entries are keyed by the tensors dropped here
-    _table_cache[key] = tab
-    return tab
+
+    def convert():
+        tab = codebook.detach().to(dtype=dtype)
+        return (tab.reshape(512, 4) if quantizer_type == "e8_d4" else tab).contiguous()
+    return _cached(_table_cache, key, codebook, convert)
 
 
 # Plain attributes the descriptor is made from; the native host path watches the buffers itself.
@@ -131,11 +124,7 @@ class EPTQLinear(nn.Module):
         out = fn(t)
         if out is t:
             return t
-        hit = _table_cache.get(key)
-        if hit is not None and hit.device == out.device and hit.dtype == out.dtype:
-            return hit
-        _table_cache[key] = out
-        return out
+        return _cached(_table_cache, (*key, out.device, out.dtype), t, lambda: out)
 
     @classmethod
     def from_quantized_data(cls, quant_data, codebook: torch.Tensor, quantizer_type: str) -> "EPTQLinear":

@@ -206,3 +206,25 @@ def test_host_extension_is_the_one_for_this_torch(built_library, monkeypatch):
     monkeypatch.setattr(torch, "__version__", "0.0.0")
     with pytest.raises(RuntimeError, match="build"):
         _lib.host()
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_layers_share_their_table_however_many_tables_there_are(built_library, kind):
+    """A cache that fills up while a model is built does not separate its layers (they run as one group launch)."""
+    qds = [make_layer(16, 8, seed=s) for s in (1, 2)]
+    base = torch.from_numpy(oracle.d4_table(1.75) if kind == "e8_d4" else oracle.e8_table(1.6)[:4096])
+    for _ in range(140):
+        tab = base.clone()
+        a, b = (EPTQLinear.from_quantized_data(qd, tab, kind) for qd in qds)
+        assert a._codebook is b._codebook and a._codebook32 is b._codebook32
+        a.to(torch.float64), b.to(torch.float64)              # what a move to a device does with the shared table
+        assert a._codebook is b._codebook
+
+
+def test_tables_are_not_mistaken_for_earlier_ones(built_library):
+    """Entries go by address and keep their source: a new codebook never meets another's copy."""
+    qd = make_layer(16, 8, seed=1)
+    for n in range(200):
+        tab = torch.from_numpy(oracle.d4_table(1.75 + 0.01 * (n % 7))).double()
+        lin = EPTQLinear.from_quantized_data(qd, tab, "e8_d4")
+        assert torch.equal(lin._codebook, tab.half().reshape(512, 4))
