@@ -313,6 +313,10 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         if (tid == 0) atomicExch(reinterpret_cast<int*>(p.counters) + (kMaxCounters - 1), static_cast<int>(EPTQ_ERR_LAUNCH));
         return;
     }
+    // Layers with group scales ran in plain stream order on the SIMT kernel, so nothing of theirs is read before the wait:
+    // weights that the previous kernel writes are seen.  (The other decode kernels read weights ahead of it and state so.)
+    // The next kernel is let in behind it for the same reason.
+    if constexpr (SCALED) asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;");
 
     const int g = lane >> 2, t = lane & 3;
@@ -404,7 +408,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     const int unit0 = warp * gridDim.x + blockIdx.x, unit_step = gridDim.x * kRowsWarps;
     CorrUnit corr = {};
     if (unit0 < p.corr_units) corr = corr_begin(p, unit0, lane);
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if constexpr (!SCALED) asm volatile("griddepcontrol.wait;" ::: "memory");
     {
         const Pos keep = pf;
         const int16_t* kq_ = qp; const __half *kx = xp, *kh = hp, *ks = sp;

@@ -85,6 +85,11 @@ enum { EPTQ_E8 = 0, EPTQ_E8D4 = 1 };
  *   bias       fp16 (8*M) or NULL.
  *   S_group    fp16 (8*M/qb_size, N) group scales or NULL (then qb_size = 0).
  *              qb_size must be a multiple of 8.
+ *
+ * The decode kernels (B <= 16) of layers without group scales start to read a layer's
+ * weights -- everything here, not x -- while the kernel before them on the stream still
+ * ends.  A program that changes weights on the stream lets that finish (an event or a
+ * stream synchronisation) before the next call.  Calls with group scales read nothing early.
  */
 typedef struct EptqLayer {
     int32_t quantizer;        /* EPTQ_E8 or EPTQ_E8D4 */

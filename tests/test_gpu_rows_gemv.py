@@ -94,3 +94,30 @@ def test_group_scales_match_oracle(kind, out, inn, qb, batch):
     ref = oracle.linear_reference(x.numpy(), W16, None if qd.bias is None else qd.bias.numpy())
     for b in range(batch):
         assert util.max_rel_err(y[b].float().cpu().numpy(), ref[b]) <= util.REL_TOL
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_group_scales_written_just_before_the_call(kind):
+    """A layer with group scales sees what the kernel before it on the stream wrote to any of its weights."""
+    import ctypes as C
+    lib = _lib.load()
+    lins, want = [], []
+    x = make_activations(1, 4096, seed=3).to(DEV)
+    for seed in (1, 2):
+        qd = make_layer(4096, 4096, seed=seed, outlier_frac=0.0, qb_size=128)
+        lins.append(EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV))
+        want.append(lins[-1](x))
+    target = EPTQLinear.from_quantized_data(make_layer(4096, 4096, seed=1, outlier_frac=0.0, qb_size=128),
+                                            torch.from_numpy(TABLES[kind]), kind).to(DEV)
+    d = target.descriptor()
+    d.h_absmax = min(lin.descriptor().h_absmax for lin in lins)               # bounds either layer's scales
+    ws = torch.zeros(lib.eptq_layer_workspace_bytes(C.byref(d), 1), dtype=torch.uint8, device=DEV)
+    ys = [torch.empty_like(want[0]) for _ in range(16)]
+    for n, y in enumerate(ys):
+        for name in ("S_group", "h", "g", "Q"):
+            getattr(target, name).copy_(getattr(lins[n % 2], name))
+        assert lib.eptq_linear_forward(C.byref(d), x.data_ptr(), y.data_ptr(), 1, ws.data_ptr(), ws.numel(),
+                                       torch.cuda.current_stream().cuda_stream) == 0
+    for n, y in enumerate(ys):
+        ref = want[n % 2].float()
+        assert torch.allclose(y.float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))
