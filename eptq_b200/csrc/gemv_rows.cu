@@ -17,8 +17,9 @@
 // rg = warp % 4); the four warps of a column group take every fourth step of the share, convert the step's
 // activations once into a shared fragment buffer (double-buffered, one 128-thread barrier per step) and each decode 8
 // Q rows.  At the end of a row tile (or of the share) the four column groups are added through shared memory and
-// the block's partial sums go to scratch with plain stores; the block (or, for a unit of corrections, warp) that takes the last
-// ticket of a row tile adds the partials in block order, so results do not depend on arrival order.
+// the block's partial sums go to scratch with plain stores; the block that takes the last
+// ticket of a row tile, for its share or for a unit of corrections, adds the partials in block order, so results do not
+// depend on arrival order.
 //
 // Group scales (SCALED; one layer, passes of 4 rows): the scale of a row group's 64 outputs multiplies x*h before the split,
 // so the four warps of a column group need different fragments and each converts its own (4 values a lane and step).
@@ -55,7 +56,7 @@ constexpr int kCorrPerTile = kTileRows / 4;
 constexpr unsigned kRowsTableAddr = 0x10000u;                   // shared-window address of the replicated E8-D4 table
 constexpr int kRowsSmemD4 = 2 * 65536 - 1024;                   // window [0x400, 0x20000)
 constexpr int kRowsSmemE8 = 232448;                             // the most a block may ask for
-constexpr unsigned kCtrlBytes = 64;
+constexpr unsigned kCtrlBytes = 128;           // last-arrival flag; from word 16 on a word per warp
 
 // Fragment buffers ([column group][2][hi, lo][NB rows][32 columns] fp16), reused for the sum over column groups.
 // With group scales every warp has its own buffers.
@@ -297,6 +298,17 @@ __device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrU
     return lane == 0 && last_arrival(p, L, rt);
 }
 
+// Row tiles whose last ticket went to a unit of corrections of this block, by warp.  With short shares a unit's chain of
+// dependent reads ends last, and the one warp that had it took 32 rounds of reads to finish the tile; the block takes two
+// (1024 x 4096 E8-D4, shares of four steps: 40.7 -> 16.5 us at 8 rows, 75.0 -> 24.7 at 16).  Not inlined: rare.
+template <int NB, int MAXL>
+__device__ __noinline__ void finish_for_units(const RowsArgs<MAXL>& p, const unsigned* done, int tid) {
+    for (int w = 0; w < kRowsWarps; ++w) {
+        const unsigned d = done[w];
+        if (d != 0u) finish_tile<NB>(p, p.L[d >> 16 & 0x7fff], d & 0xffff, tid, kRowsThreads);
+    }
+}
+
 template <int KIND, int NB, int MAXL, bool SCALED>
 __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid_constant__ RowsArgs<MAXL> p) {
     constexpr int RING = ring_steps(NB);
@@ -423,7 +435,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     // The first unit's ticket is looked at behind the main loop (its round trip costs nothing there).
     bool corr_last = false;
     if (unit0 < p.corr_units) corr_last = corr_finish<KIND, NB, SCALED>(p, corr, lane);
-    const int corr_l = corr.l, corr_rt = corr.qt / kCorrPerTile;
+    const unsigned corr_tile = 1u << 31 | static_cast<unsigned>(corr.l) << 16 | static_cast<unsigned>(corr.qt / kCorrPerTile);
     for (int u = unit0 + unit_step; u < p.corr_units; u += unit_step) {
         const CorrUnit c = corr_begin(p, u, lane);
         const bool last = corr_finish<KIND, NB, SCALED>(p, c, lane);
@@ -608,7 +620,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
             cur.k += kColGroups;
         }
     }
-    if (__any_sync(0xffffffffu, corr_last)) finish_tile<NB>(p, p.L[corr_l], corr_rt, lane, 32);
+    if (__syncthreads_or(corr_last)) {
+        if (lane == 0) flag[16 + warp] = corr_last ? corr_tile : 0u;
+        __syncthreads();
+        finish_for_units<NB>(p, flag + 16, tid);
+    }
 }
 
 struct RowsPlan {

@@ -121,3 +121,14 @@ def test_group_scales_written_just_before_the_call(kind):
     for n, y in enumerate(ys):
         ref = want[n % 2].float()
         assert torch.allclose(y.float(), ref, rtol=2e-3, atol=2e-3 * float(ref.abs().max()))
+
+
+@pytest.mark.parametrize("kind,out,inn,frac", [("e8_d4", 1024, 4096, 0.002), ("e8_d4", 512, 4096, 0.02), ("e8_lattice", 1024, 8192, 0.002)])
+@pytest.mark.parametrize("batch", [3, 8, 16])
+def test_rows_few_tiles(kind, out, inn, frac, batch):
+    """Many blocks with short shares per row tile: a unit of corrections often takes the tile's last ticket."""
+    qds, lins = layers_of(kind, [(out, inn)], (frac,))
+    x = make_activations(batch, inn, seed=batch)
+    ys = [lins[0](x.to(DEV)) for _ in range(20)]
+    check(kind, qds, [x], ys[:1])
+    assert all(torch.equal(y, ys[0]) for y in ys)
