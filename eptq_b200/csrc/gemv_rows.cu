@@ -23,8 +23,15 @@
 //
 // Group scales (SCALED; one layer, passes of 4 rows): the scale of a row group's 64 outputs multiplies x*h before the split,
 // so the four warps of a column group need different fragments and each converts its own (4 values a lane and step).
-// Taken for qb_size % 64 == 0; the SIMT kernel, which multiplies in its inner loop, stays for the rest
-// (14336 x 4096 E8-D4, scales per 128 rows, 1 row: 34.8 -> 19.5 us).
+// The SIMT kernel holds x*h*S and its products in 32 bits, and the split here loses none of that: each batch row is scaled
+// by a power of two from its own max|x| (a pass over the rows while the table arrives), so that its values use the upper
+// binades of fp16; the remainder is kept times 2^11; and codewords are lattice coordinates, small whole or half numbers,
+// whose products with 11-bit parts the tensor core adds without loss.  Error of the sums against 64 bits, x of 1e-4 to 10,
+// four shapes up to 4096 x 14336: log-normal S and h of sigma 0.1 and 0.25 1.2e-7 (SIMT kernel 1.4e-7), 0.5 and 0.3 1.3e-7
+// (1.4e-7), 1.2 and 0.1 2.4e-7 (1.5e-7: the tensor core cuts where the other rounds); without the three up to 4e-2.
+// Time with them, 14336 x 4096 at 1 row: E8-D4 19.6 -> 21.3 us, E8 25.4 -> 26.3 us.
+// Taken for qb_size % 64 == 0 where it is the faster one (rows_scaled_supported); the SIMT kernel, which multiplies in its
+// inner loop, stays for the rest.
 //
 // Critical blocks: while the table arrives, the warps of the launch walk the CSR tables in units of 4 Q rows (at most a
 // unit or two per warp for the fractions in use) and store sum (O - code[65535])*h*x to a slot of their own that the
@@ -83,7 +90,7 @@ struct RowsLayer {
     int corr_tile;          // correction units per row tile: 8, or 0 for a layer without critical blocks
     int qb_rows;            // Q rows per scale group, 0 without group scales
     const __half* S;
-    float x_scale;          // power of two, <= 1 / max|h| (/ max|S|)
+    float x_scale;          // power of two, <= 1 / max|h| (/ max|S|; then times the batch row's own power of two)
     float x_inv_scale;
 };
 
@@ -94,6 +101,7 @@ struct RowsArgs {
     const unsigned* packed;
     unsigned* counters;     // zero on entry, zero again on exit
     float* partial;         // [block + tile][NB][256] main partials, then [tile][NB][256] corrections
+    float code_unit;        // group scales, E8-D4: table16 = lattice coordinate * code_unit
     unsigned W;             // steps
     int G;                  // blocks with a share
     int tiles;
@@ -123,6 +131,26 @@ __device__ __forceinline__ uint4 ldg_once(const void* p) {
 __device__ __forceinline__ void split_half(float v, __half& hi, __half& lo) {
     hi = __float2half_rn(v);
     lo = __float2half_rn(v - __half2float(hi));
+}
+// x * s = hi + lo * 2^-11 with one rounding of the remainder (a fused multiply-add forms it): 22 bits and the sign while hi
+// is normal, and for |x * s| <= 2^15 a remainder times 2^11 is at most 2^15 too.
+constexpr float kLoScale = 2048.f;
+__device__ __forceinline__ void split_product(float x, float s, __half& hi, __half& lo) {
+    hi = __float2half_rn(x * s);
+    lo = __float2half_rn(fmaf(x, s, -__half2float(hi)) * kLoScale);
+}
+// 2^n, -126 <= n <= 127
+__device__ __forceinline__ float exp2i(int n) { return __int_as_float((127 + n) << 23); }
+// Biased fp16 exponent e of a row's largest |x| (bits): |x| < 2^(e-14).  Infinities and NaN count as the largest finite.
+__device__ __forceinline__ int row_exponent(unsigned bits) { return min(max(static_cast<int>(bits >> 10), 1), 30); }
+constexpr int kRowTop = 29;                 // a row's values times 2^(kRowTop - e) stay below 2^15
+
+// A coordinate of the E8-D4 lattice from its fp16 table entry: the rounding of the entry is far less than half a step.
+__device__ __forceinline__ float lattice(__half code, float inv_unit) { return rintf(__half2float(code) * inv_unit); }
+__device__ __forceinline__ unsigned lattice2(unsigned codes, float inv_unit) {
+    const __half2 c = *reinterpret_cast<const __half2*>(&codes);
+    const __half2 v = __floats2half2_rn(lattice(__low2half(c), inv_unit), lattice(__high2half(c), inv_unit));
+    return *reinterpret_cast<const unsigned*>(&v);
 }
 
 // Packed E8 entry -> fp16 pairs of dims (0,1), (2,3), (4,5), (6,7): the layout and the arithmetic are stated at
@@ -247,6 +275,10 @@ __device__ __forceinline__ bool corr_finish(const RowsArgs<MAXL>& p, const CorrU
         const float2 c01 = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
         const float2 c23 = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
         cstar[0] = c01.x; cstar[1] = c01.y; cstar[2] = c23.x; cstar[3] = c23.y;
+        if constexpr (SCALED) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cstar[k] = rintf(cstar[k] * (1.f / p.code_unit)) * p.code_unit;
+        }
     }
     const RowsLayer& L = p.L[c.l];
     const int rt = c.qt / kCorrPerTile, sub = lane & 7;
@@ -325,10 +357,35 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         if (tid == 0) atomicExch(reinterpret_cast<int*>(p.counters) + (kMaxCounters - 1), static_cast<int>(EPTQ_ERR_LAUNCH));
         return;
     }
+    unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB, SCALED));
+    unsigned* const row_max = flag + 4;                        // group scales: bits of max|x| of the four batch rows
+    auto fill_table = [&]() {
+        if constexpr (KIND == EPTQ_E8) {
+            const unsigned dst0 = base + e8_table_offset(NB, SCALED);
+            const char* src0 = reinterpret_cast<const char*>(p.packed);
+            for (unsigned off = tid * 16u; off < e8_resident(NB, SCALED) * 4u; off += kRowsThreads * 16u)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst0 + off), "l"(src0 + off) : "memory");
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        } else {
+            // entry order follows the raw stored bits (true index ^ 0x100 on 9 bits), 16 copies of 8 bytes per entry
+            unsigned char* tab = smem_raw + (kRowsTableAddr - base);
+            static_assert(kRowsThreads == 512, "one table entry per thread");
+            uint2 v = __ldg(p.table16 + (tid ^ 0x100));
+            if constexpr (SCALED) { const float inv = 1.f / p.code_unit; v.x = lattice2(v.x, inv); v.y = lattice2(v.y, inv); }
+            const uint4 vv = make_uint4(v.x, v.y, v.x, v.y);
+    #pragma unroll
+            for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tab + tid * 128 + ((c + tid) & 7) * 16) = vv;
+        }
+    };
     // Layers with group scales ran in plain stream order on the SIMT kernel, so nothing of theirs is read before the wait:
     // weights that the previous kernel writes are seen.  (The other decode kernels read weights ahead of it and state so.)
-    // The next kernel is let in behind it for the same reason.
-    if constexpr (SCALED) asm volatile("griddepcontrol.wait;" ::: "memory");
+    // The next kernel is let in behind it for the same reason.  The codebook, made once for all layers, comes ahead.
+    if constexpr (SCALED) {
+        if (tid < 4) row_max[tid] = 0u;
+        fill_table();
+        __syncthreads();
+        asm volatile("griddepcontrol.wait;" ::: "memory");
+    }
     asm volatile("griddepcontrol.launch_dependents;");
 
     const int g = lane >> 2, t = lane & 3;
@@ -402,20 +459,14 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         if (pf.l < p.n_layers) { ring[i].q = ldg_once(qp); load_cols(hp, ring[i].h); if constexpr (SCALED) load_cols(sp, ring[i].s); next(); }
     }
 
-    if constexpr (KIND == EPTQ_E8) {
-        const unsigned dst0 = base + e8_table_offset(NB, SCALED);
-        const char* src0 = reinterpret_cast<const char*>(p.packed);
-        for (unsigned off = tid * 16u; off < e8_resident(NB, SCALED) * 4u; off += kRowsThreads * 16u)
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(dst0 + off), "l"(src0 + off) : "memory");
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    } else {
-        // entry order follows the raw stored bits (true index ^ 0x100 on 9 bits), 16 copies of 8 bytes per entry
-        unsigned char* tab = smem_raw + (kRowsTableAddr - base);
-        static_assert(kRowsThreads == 512, "one table entry per thread");
-        const uint2 v = __ldg(p.table16 + (tid ^ 0x100));
-        const uint4 vv = make_uint4(v.x, v.y, v.x, v.y);
+    if constexpr (!SCALED) fill_table();
+    // group scales: the batch rows' values whose largest is sought, this thread's first 8 columns of each
+    uint4 part[SCALED ? 4 : 1];
+    const bool has_part = SCALED && tid * 8 < p.L[0].N;
+    auto row_cols = [&](int b, int col) { return ldg128(p.L[0].x + static_cast<size_t>(b) * p.L[0].N + col); };
+    if constexpr (SCALED) {
 #pragma unroll
-        for (int c = 0; c < 8; ++c) *reinterpret_cast<uint4*>(tab + tid * 128 + ((c + tid) & 7) * 16) = vv;
+        for (int b = 0; b < 4; ++b) part[b] = has_part && b < p.B ? row_cols(b, tid * 8) : make_uint4(0, 0, 0, 0);
     }
     const int unit0 = warp * gridDim.x + blockIdx.x, unit_step = gridDim.x * kRowsWarps;
     CorrUnit corr = {};
@@ -430,6 +481,24 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         for (int i = 0; i < RING; ++i)
             if (pf.l < p.n_layers) { if (xlive) load_cols(xp, ring[i].x); next(); }
         pf = keep; qp = kq_; xp = kx; hp = kh; sp = ks;
+    }
+
+    if constexpr (SCALED) {
+        auto largest = [](const uint4& v) {
+            return __vmaxu2(__vmaxu2(v.x & 0x7fff7fffu, v.y & 0x7fff7fffu), __vmaxu2(v.z & 0x7fff7fffu, v.w & 0x7fff7fffu));
+        };
+        unsigned top[4];
+#pragma unroll
+        for (int b = 0; b < 4; ++b) top[b] = largest(part[b]);
+        for (int i = (tid + kRowsThreads) * 8; i < p.L[0].N; i += kRowsThreads * 8)
+#pragma unroll
+            for (int b = 0; b < 4; ++b)
+                if (b < p.B) top[b] = __vmaxu2(top[b], largest(row_cols(b, i)));
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const unsigned m = __reduce_max_sync(0xffffffffu, max(top[b] & 0xffffu, top[b] >> 16));
+            if (lane == 0) atomicMax(row_max + b, m);
+        }
     }
 
     // The first unit's ticket is looked at behind the main loop (its round trip costs nothing there).
@@ -447,10 +516,17 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
 
     const unsigned area = base;                                // fragment buffers / sums over column groups
     unsigned char* const area_p = smem_raw;
-    unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB, SCALED));
     const unsigned my_buf = (SCALED ? warp : kq) * 2 * kBuf;
     const unsigned wr_off = my_buf + ((xcol >> 2) & 1) * kHalf + xrow * 32 + (xcol >> 3) * 8 + (xcol & 3) * 2;
     const unsigned rd_addr = area + my_buf + g * 32 + t * 8;
+    // this thread's rows: the one it converts, and the two it stores (behind `lo` of the same row pair where t >= 2)
+    float row_up = 1.f, row_down[2] = {1.f, 1.f};
+    if constexpr (SCALED) {
+        row_up = exp2i(kRowTop - row_exponent(row_max[xrow]));
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+            row_down[e] = exp2i(row_exponent(row_max[2 * (t & 1) + e]) - kRowTop) * (t >= 2 ? 1.f / kLoScale : 1.f);
+    }
     const unsigned lane_tab = 8u * (lane & 15) | kRowsTableAddr;
     const unsigned tbase = base + e8_table_offset(NB, SCALED);
 
@@ -486,11 +562,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         }
         if (kq == 0) {
             float* dst = p.partial + (static_cast<size_t>(blockIdx.x + L.tile0 + cur.rt) * NB) * kTileOut + (rg * 8 + g) * 8;
-            const float inv = L.x_inv_scale;
 #pragma unroll
             for (int i = 0; i < BT; ++i)
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {                  // batch rows 2t and 2t+1 of the column tile
+                    const float inv = SCALED ? L.x_inv_scale * row_down[e] : L.x_inv_scale;
                     float v[8];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) { v[2 * j] = acc[i][j][e] * inv; v[2 * j + 1] = acc[i][j][2 + e] * inv; }
@@ -544,15 +620,20 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         const uint4 q = in.q;
         const unsigned qw[4] = {q.x, q.y, q.z, q.w};
         {
-            const float sc = p.L[cur.l].x_scale;
+            const float sc = SCALED ? p.L[cur.l].x_scale * row_up : p.L[cur.l].x_scale;
             __half hi[XC], lo[XC];
 #pragma unroll
             for (int e = 0; e < XC; ++e) {
                 const unsigned short xb = static_cast<unsigned short>(in.x[e >> 1] >> (16 * (e & 1)));
                 const unsigned short hb = static_cast<unsigned short>(in.h[e >> 1] >> (16 * (e & 1)));
                 float hx = __half2float(__ushort_as_half(hb)) * sc;
-                if constexpr (SCALED) hx *= __half2float(__ushort_as_half(static_cast<unsigned short>(in.s[e >> 1] >> (16 * (e & 1)))));
-                split_half(__half2float(__ushort_as_half(xb)) * hx, hi[e], lo[e]);
+                const float xv = __half2float(__ushort_as_half(xb));
+                if constexpr (SCALED) {                        // h * S is exact: 22 bits
+                    hx *= __half2float(__ushort_as_half(static_cast<unsigned short>(in.s[e >> 1] >> (16 * (e & 1)))));
+                    split_product(xv, hx, hi[e], lo[e]);
+                } else {
+                    split_half(xv * hx, hi[e], lo[e]);
+                }
             }
             unsigned char* w = area_p + wr_off + par * kBuf;
             if constexpr (XC == 4) {
@@ -689,6 +770,7 @@ int launch_sized(const RowsPlan& plan, const EptqLayer* layers, int n, const uin
     a.packed = e8 ? layers[0].table_packed : nullptr;
     a.counters = reinterpret_cast<unsigned*>(workspace);
     a.partial = reinterpret_cast<float*>(reinterpret_cast<char*>(workspace) + kPartialOffset);
+    a.code_unit = layers[0].table8_scale;
     a.W = plan.W; a.G = plan.G; a.tiles = plan.tiles;
     a.n_layers = n;
     a.B = B;
@@ -717,7 +799,7 @@ int launch_sized(const RowsPlan& plan, const EptqLayer* layers, int n, const uin
         int e = 0;
         std::frexp(std::fabs(L.h_absmax), &e);            // h_absmax = m * 2^e, m in [0.5, 1)  =>  2^-e <= 1/h_absmax
         R.x_scale = std::ldexp(1.0f, -e);
-        R.x_inv_scale = std::ldexp(1.0f, e) * (e8 ? L.table_packed_scale : 1.0f);
+        R.x_inv_scale = std::ldexp(1.0f, e) * (e8 ? L.table_packed_scale : L.S_group != nullptr ? L.table8_scale : 1.0f);
         step0 += R.row_tiles * R.ns;
         tile0 += R.row_tiles;
         corr0 += R.row_tiles * R.corr_tile;
@@ -754,7 +836,7 @@ bool rows_scaled_supported(const EptqLayer& L, int B) {
            (L.N % 32) == 0 && aligned16(L.Q) && aligned16(L.h) && aligned16(L.g) && aligned16(L.S_group) &&
            (L.bias == nullptr || aligned16(L.bias)) && (L.n_masked == 0 || aligned16(L.O_vals)) &&
            (L.quantizer == EPTQ_E8 ? L.table_packed != nullptr && aligned16(L.table_packed) && L.table_packed_scale > 0.f
-                                   : L.table16 != nullptr && aligned16(L.table16));
+                                   : L.table16 != nullptr && aligned16(L.table16) && L.table8 != nullptr && L.table8_scale > 0.f);
 }
 
 // Passes of four rows, the scratch of rows_workspace_bytes(&L, 1, 4, n_sms).

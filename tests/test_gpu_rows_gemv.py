@@ -132,3 +132,40 @@ def test_rows_few_tiles(kind, out, inn, frac, batch):
     ys = [lins[0](x.to(DEV)) for _ in range(20)]
     check(kind, qds, [x], ys[:1])
     assert all(torch.equal(y, ys[0]) for y in ys)
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("spread_s,spread_h", [(0.1, 0.25), (1.2, 0.1)])
+def test_group_scales_keep_32_bits(kind, spread_s, spread_h):
+    """Activations of any size, each batch row its own, and scales that differ a thousandfold between groups.  The sums are
+    compared beyond fp16 by a second call whose bias cancels the first one's result."""
+    out, inn, qb = 4096, 6176, 128
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    qd = make_layer(out, inn, seed=4, outlier_frac=0.004, qb_size=qb, device=DEV, scale_sigma=spread_h)
+    qd.S_group = torch.exp(spread_s * torch.randn(qd.S_group.shape, generator=gen, device=DEV)).half()
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]).to(DEV), kind)
+    code = lin._codebook32.double()
+    idx = lin.Q.long() + 32768
+    if kind == "e8_d4":
+        W = torch.cat([code[(idx >> 14) * 128 + ((idx >> 7) & 127)], code[(idx >> 14) * 128 + (idx & 127)]], -1)
+    else:
+        W = code[idx.clamp(max=code.shape[0] - 1)]
+    W = W * lin.S_group.double().repeat_interleave(qb // 8, 0)[:, :, None]
+    W[idx == 65535] = lin.O_vals.double()
+    W = (W * lin.h.double()[None, :, None]).permute(0, 2, 1).reshape(out, inn)
+    for size in (30.0, 1.0, 1e-2, 1e-3, 1e-4):
+        x = (size * torch.randn((1, inn), generator=gen, device=DEV)).half()
+        sums = (x.double() @ W.T)[0]
+        groups = sums.view(-1, qb)
+        lin.g = torch.exp2(-torch.log2(groups.abs().amax(1)).ceil()).clamp(2.0 ** -14, 32768.0).repeat_interleave(qb).half()
+        lin.bias = None
+        before = _lib.load().eptq_kernel_launch_count(1)
+        # other rows of other sizes beside it must not matter
+        first = lin(torch.cat([x, 100 * x.clamp(-600, 600), x * 0.01]))[0]
+        lin.bias = -first
+        both = first.double() + lin(x)[0].double()
+        assert _lib.load().eptq_kernel_launch_count(1) - before == 2                # the multi-row kernel took both
+        want = sums * lin.g.double()
+        rms = want.view(-1, qb).pow(2).mean(1).sqrt().repeat_interleave(qb)
+        # fp32 sums of 6176 products: below 1e-6 of a group's rms; the second result is fp16 of a difference below 2^-11
+        assert float(((both - want).abs() / (rms + want.abs())).max()) <= 4e-6
