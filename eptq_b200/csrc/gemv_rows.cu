@@ -63,7 +63,10 @@ constexpr int kCorrPerTile = kTileRows / 4;
 constexpr unsigned kRowsTableAddr = 0x10000u;                   // shared-window address of the replicated E8-D4 table
 constexpr int kRowsSmemD4 = 2 * 65536 - 1024;                   // window [0x400, 0x20000)
 constexpr int kRowsSmemE8 = 232448;                             // the most a block may ask for
-constexpr unsigned kCtrlBytes = 128;           // last-arrival flag; from word 16 on a word per warp
+// Control words: 0 last-arrival flag, 1 finished tiles, 4..7 row maxima, 16..31 a word per warp, 32.. the finished tiles.  Of
+// those a block has at most 16 from units of corrections and 9 from its share, which touches at most tiles / G + 2 (148
+// blocks, or shares of up to seven steps: plan_rows).
+constexpr unsigned kCtrlBytes = 256;
 
 // Fragment buffers ([column group][2][hi, lo][NB rows][32 columns] fp16), reused for the sum over column groups.
 // With group scales every warp has its own buffers.
@@ -231,6 +234,43 @@ __device__ __forceinline__ void finish_tile(const RowsArgs<MAXL>& p, const RowsL
     }
 }
 
+// `row_max`: bits of max|x| of the four batch rows.
+__device__ __forceinline__ bool any_nonfinite(const unsigned* row_max) {
+    return max(max(row_max[0], row_max[1]), max(row_max[2], row_max[3])) >= 0x7c00u;
+}
+// The outputs, in the tiles a block finished, of batch rows with an infinity or a NaN in a layer with group scales.  The
+// tensor core multiplies every column by every codeword, a critical block's stand-in and zero coordinates among them, and
+// the split would subtract infinities; this is the SIMT kernel's arithmetic, which does neither.  Slow, and rare.
+template <int KIND, int MAXL>
+__device__ __noinline__ void finish_nonfinite(const RowsArgs<MAXL>& p, const unsigned* tiles, unsigned n_tiles, int tid, const unsigned* row_max) {
+    const RowsLayer& L = p.L[0];
+    for (int i = tid; i < static_cast<int>(n_tiles) * p.B * kTileOut; i += kRowsThreads) {
+        const int b = i / kTileOut % p.B, rt = static_cast<int>(tiles[i / kTileOut / p.B]);
+        const int dim = i % 8, row = rt * kTileRows + i % kTileOut / 8;
+        if (row >= L.M || row_max[b] < 0x7c00u) continue;
+        const __half* x = L.x + static_cast<size_t>(b) * L.N;
+        const __half* S = L.S + static_cast<size_t>(row / L.qb_rows) * L.N;
+        const __half* table = reinterpret_cast<const __half*>(p.table16);
+        int block = __ldg(L.O_row_ptr + row);
+        float sum = 0.f;
+        for (int k = 0; k < L.N; ++k) {
+            const unsigned idx = (static_cast<unsigned>(L.Q[static_cast<size_t>(row) * L.N + k]) & 0xffffu) ^ 0x8000u;
+            float v = __half2float(L.h[k]), code;
+            if (idx == kMarkerIndex) {
+                code = __half2float(L.O_vals[static_cast<size_t>(block++) * 8 + dim]);
+            } else {
+                v *= __half2float(S[k]);
+                code = __half2float(KIND == EPTQ_E8 ? table[static_cast<size_t>(idx) * 8 + dim]
+                                                    : table[(((idx >> 7) & 0x180u) | ((dim >= 4 ? idx : idx >> 7) & 127u)) * 4 + dim % 4]);
+            }
+            sum = fmaf(code, v * __half2float(x[k]), sum);
+        }
+        const int o = row * 8 + dim;
+        L.y[static_cast<size_t>(b) * 8 * L.M + o] =
+            __float2half_rn(fmaf(sum, __half2float(L.g[o]), L.bias != nullptr ? __half2float(L.bias[o]) : 0.f));
+    }
+}
+
 template <int MAXL>
 __device__ __forceinline__ bool last_arrival(const RowsArgs<MAXL>& p, const RowsLayer& L, int rt) {
     unsigned ticket;
@@ -359,6 +399,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     }
     unsigned* const flag = reinterpret_cast<unsigned*>(smem_raw + area_bytes(NB, SCALED));
     unsigned* const row_max = flag + 4;                        // group scales: bits of max|x| of the four batch rows
+    unsigned* const finished = flag + 32;                      // group scales: flag[1] row tiles that this block finished
     auto fill_table = [&]() {
         if constexpr (KIND == EPTQ_E8) {
             const unsigned dst0 = base + e8_table_offset(NB, SCALED);
@@ -382,6 +423,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
     // The next kernel is let in behind it for the same reason.  The codebook, made once for all layers, comes ahead.
     if constexpr (SCALED) {
         if (tid < 4) row_max[tid] = 0u;
+        if (tid == 0) flag[1] = 0u;
         fill_table();
         __syncthreads();
         asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -499,13 +541,14 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
             const unsigned m = __reduce_max_sync(0xffffffffu, max(top[b] & 0xffffu, top[b] >> 16));
             if (lane == 0) atomicMax(row_max + b, m);
         }
+        __syncthreads();                                       // a unit of corrections may finish a tile from here on
     }
 
     // The first unit's ticket is looked at behind the main loop (its round trip costs nothing there).
     bool corr_last = false;
     if (unit0 < p.corr_units) corr_last = corr_finish<KIND, NB, SCALED>(p, corr, lane);
     const unsigned corr_tile = 1u << 31 | static_cast<unsigned>(corr.l) << 16 | static_cast<unsigned>(corr.qt / kCorrPerTile);
-    for (int u = unit0 + unit_step; u < p.corr_units; u += unit_step) {
+    for (int u = unit0 + unit_step; !SCALED && u < p.corr_units; u += unit_step) {
         const CorrUnit c = corr_begin(p, u, lane);
         const bool last = corr_finish<KIND, NB, SCALED>(p, c, lane);
         if (__any_sync(0xffffffffu, last)) finish_tile<NB>(p, p.L[c.l], c.qt / kCorrPerTile, lane, 32);
@@ -591,7 +634,11 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         __syncthreads();
         if (tid == 0) *flag = last_arrival(p, L, cur.rt) ? 1u : 0u;
         __syncthreads();
-        if (*flag != 0u) finish_tile<NB>(p, L, cur.rt, tid, kRowsThreads);
+        if (*flag != 0u) {
+            finish_tile<NB>(p, L, cur.rt, tid, kRowsThreads);
+            if constexpr (SCALED)
+                if (tid == 0) finished[flag[1]++] = cur.rt;
+        }
     };
     // Segment after the current one; false when the block's share is done.
     auto next_segment = [&]() {
@@ -705,7 +752,13 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         if (lane == 0) flag[16 + warp] = corr_last ? corr_tile : 0u;
         __syncthreads();
         finish_for_units<NB>(p, flag + 16, tid);
+        if constexpr (SCALED) {
+            if (lane == 0 && corr_last) finished[atomicAdd(flag + 1, 1u)] = corr_tile & 0xffffu;
+            __syncthreads();
+        }
     }
+    if constexpr (SCALED)                                      // behind a barrier: the list and the outputs are written
+        if (any_nonfinite(row_max)) finish_nonfinite<KIND>(p, finished, flag[1], tid, row_max);
 }
 
 struct RowsPlan {
@@ -832,7 +885,8 @@ int launch_gemv_rows(const EptqLayer* layers, int n, const uint16_t* const* xs, 
 
 // One layer with group scales that are constant over 64 outputs; -h_absmax = max|h| * max|S_group| bounds x*h*S.
 bool rows_scaled_supported(const EptqLayer& L, int B) {
-    return L.S_group != nullptr && L.qb_size > 0 && (L.qb_size % 64) == 0 && L.h_absmax < 0.f && std::isfinite(L.h_absmax) && B >= 1 && B <= kGemmMinBatch &&
+    RowsPlan plan;                               // one unit of corrections per warp at most
+    return plan_rows(&L, 1, 4, kSms, plan) && plan.tiles * kCorrPerTile <= plan.G * kRowsWarps && L.S_group != nullptr && L.qb_size > 0 && (L.qb_size % 64) == 0 && L.h_absmax < 0.f && std::isfinite(L.h_absmax) && B >= 1 && B <= kGemmMinBatch &&
            (L.N % 32) == 0 && aligned16(L.Q) && aligned16(L.h) && aligned16(L.g) && aligned16(L.S_group) &&
            (L.bias == nullptr || aligned16(L.bias)) && (L.n_masked == 0 || aligned16(L.O_vals)) &&
            (L.quantizer == EPTQ_E8 ? L.table_packed != nullptr && aligned16(L.table_packed) && L.table_packed_scale > 0.f

@@ -169,3 +169,37 @@ def test_group_scales_keep_32_bits(kind, spread_s, spread_h):
         rms = want.view(-1, qb).pow(2).mean(1).sqrt().repeat_interleave(qb)
         # fp32 sums of 6176 products: below 1e-6 of a group's rms; the second result is fp16 of a difference below 2^-11
         assert float(((both - want).abs() / (rms + want.abs())).max()) <= 4e-6
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+@pytest.mark.parametrize("batch", [1, 4, 6])
+def test_group_scales_infinities(kind, batch):
+    """An infinity or a NaN in the activations gives what the SIMT kernel gives, also where the column is a critical block
+    of some rows or a codeword coordinate is zero; rows without one are not touched."""
+    import ctypes as C
+    out, inn = 4096, 6176
+    qd = make_layer(out, inn, seed=6, outlier_frac=0.004, bias=True, qb_size=128)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV)
+    lib = _lib.load()
+    col = int(lin.O_col[int(lin.O_row_ptr[40])])                         # a critical block of Q row 40
+    for places in ([(0, 17, float("inf"))], [(0, col, -float("inf"))], [(batch - 1, 5, float("inf")), (batch - 1, 6000, float("inf"))],
+                   [(batch // 2, col, float("nan"))], [(0, 1, float("inf")), (0, 2, -float("inf"))]):
+        x = make_activations(batch, inn, seed=3).to(DEV)
+        clean = lin(x)
+        for b, c, v in places:
+            x[b, c] = v
+        before = lib.eptq_kernel_launch_count(1)
+        y = lin(x)
+        assert lib.eptq_kernel_launch_count(1) - before == (batch + 3) // 4
+        d = lin.descriptor()
+        d.h_absmax = 0.0                                                 # no bound: the SIMT kernel
+        ws = torch.zeros(lib.eptq_layer_workspace_bytes(C.byref(d), batch), dtype=torch.uint8, device=DEV)
+        ref = torch.empty_like(y)
+        assert lib.eptq_linear_forward(C.byref(d), x.data_ptr(), ref.data_ptr(), batch, ws.data_ptr(), ws.numel(),
+                                       torch.cuda.current_stream().cuda_stream) == 0
+        assert torch.equal(y.isnan(), ref.isnan()) and torch.equal(y.isposinf(), ref.isposinf()) and torch.equal(y.isneginf(), ref.isneginf())
+        hit = {b for b, _, _ in places}
+        for b in range(batch):
+            assert bool(y[b].isfinite().all()) != (b in hit)
+            if b not in hit:
+                assert torch.equal(y[b], clean[b])
