@@ -883,10 +883,21 @@ int launch_gemv_rows(const EptqLayer* layers, int n, const uint16_t* const* xs, 
                                : launch_sized<kRowsMaxLayers>(plan, layers, n, xs, ys, B, workspace, stream);
 }
 
+// Where passes of four rows beat the SIMT kernel.  They cost a fixed part (table, row maxima, partial sums) once per four
+// rows, that one its arithmetic per row, and few row tiles leave blocks with short shares.  E8-D4 / E8, scales per 128 rows,
+// SIMT against this, us: 4096 x 4096 (2.1 M indices) 1 row 12.0, 15.5 / 14.3, 17.6; 4 rows 19.7, 15.8 / 22.9, 18.1; 8 rows
+// 39.7, 31.1 / 51.8, 35.6; 16 rows 51.5, 62.0 / 69.3, 70.7.  5120 x 5120 (3.3 M) 1 row 21.1, 17.6 / 23.6, 20.2; 16 rows 74.1,
+// 70.2 / 107, 81.  Few tiles: 2048 x 8192 (2.1 M) 4 rows 19.7, 17.6 / 23.0, 19.2; 12 rows 50.2, 52.1; 2048 x 14336 (3.7 M) 1
+// row 17.3, 20.6 / 21.3, 23.1; 2432 x 14336 (4.4 M) 1 row 23.3, 21.3 / 24.5, 24.1; 1024 x 16384 (2.1 M) 4 rows 16.3, 23.4.
+static bool rows_scaled_faster(long long M, long long N, int B) {
+    if (M >= 288 && M * N >= 3LL << 20) return true;
+    return B >= 3 && B <= 8 && M >= 256 && M * N >= 2LL << 20;
+}
+
 // One layer with group scales that are constant over 64 outputs; -h_absmax = max|h| * max|S_group| bounds x*h*S.
 bool rows_scaled_supported(const EptqLayer& L, int B) {
     RowsPlan plan;                               // one unit of corrections per warp at most
-    return plan_rows(&L, 1, 4, kSms, plan) && plan.tiles * kCorrPerTile <= plan.G * kRowsWarps && L.S_group != nullptr && L.qb_size > 0 && (L.qb_size % 64) == 0 && L.h_absmax < 0.f && std::isfinite(L.h_absmax) && B >= 1 && B <= kGemmMinBatch &&
+    return rows_scaled_faster(L.M, L.N, B) && plan_rows(&L, 1, 4, kSms, plan) && plan.tiles * kCorrPerTile <= plan.G * kRowsWarps && L.S_group != nullptr && L.qb_size > 0 && (L.qb_size % 64) == 0 && L.h_absmax < 0.f && std::isfinite(L.h_absmax) && B >= 1 && B <= kGemmMinBatch &&
            (L.N % 32) == 0 && aligned16(L.Q) && aligned16(L.h) && aligned16(L.g) && aligned16(L.S_group) &&
            (L.bias == nullptr || aligned16(L.bias)) && (L.n_masked == 0 || aligned16(L.O_vals)) &&
            (L.quantizer == EPTQ_E8 ? L.table_packed != nullptr && aligned16(L.table_packed) && L.table_packed_scale > 0.f

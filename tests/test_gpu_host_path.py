@@ -55,8 +55,8 @@ def test_calls_follow_changed_buffers(kind, tokens):
 
 @pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
 def test_group_scales_follow_changed_buffers(kind):
-    lin = layer(kind, out=4096, inn=2048, qb_size=128)
-    x = make_activations(1, 2048, seed=9, device=DEV)
+    lin = layer(kind, out=4096, inn=6176, qb_size=128)
+    x = make_activations(1, 6176, seed=9, device=DEV)
     lin.g.mul_(2.0 ** -12)
     for change in (lambda: None, lambda: lin.S_group.mul_(4096), lambda: setattr(lin, "S_group", lin.S_group / 512)):
         change()

@@ -76,7 +76,7 @@ def test_small_scratch_takes_passes_of_two_rows(kind):
 
 
 @pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
-@pytest.mark.parametrize("out,inn,qb,batch", [(2048, 4096, 128, 1), (1536, 5504, 512, 3), (4160, 2080, 64, 5), (2048, 4128, 2048, 16)])
+@pytest.mark.parametrize("out,inn,qb,batch", [(4096, 6176, 128, 1), (5120, 5504, 512, 3), (4160, 4128, 64, 5), (4096, 6176, 2048, 16)])
 def test_group_scales_match_oracle(kind, out, inn, qb, batch):
     """Group scales in passes of four rows; scales that span a factor of about a thousand."""
     from eptq_b200.kernels import h_absmax
@@ -102,12 +102,12 @@ def test_group_scales_written_just_before_the_call(kind):
     import ctypes as C
     lib = _lib.load()
     lins, want = [], []
-    x = make_activations(1, 4096, seed=3).to(DEV)
+    x = make_activations(1, 6176, seed=3).to(DEV)
     for seed in (1, 2):
-        qd = make_layer(4096, 4096, seed=seed, outlier_frac=0.0, qb_size=128)
+        qd = make_layer(4096, 6176, seed=seed, outlier_frac=0.0, qb_size=128)
         lins.append(EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES[kind]), kind).to(DEV))
         want.append(lins[-1](x))
-    target = EPTQLinear.from_quantized_data(make_layer(4096, 4096, seed=1, outlier_frac=0.0, qb_size=128),
+    target = EPTQLinear.from_quantized_data(make_layer(4096, 6176, seed=1, outlier_frac=0.0, qb_size=128),
                                             torch.from_numpy(TABLES[kind]), kind).to(DEV)
     d = target.descriptor()
     d.h_absmax = min(lin.descriptor().h_absmax for lin in lins)               # bounds either layer's scales
@@ -203,3 +203,22 @@ def test_group_scales_infinities(kind, batch):
             assert bool(y[b].isfinite().all()) != (b in hit)
             if b not in hit:
                 assert torch.equal(y[b], clean[b])
+
+
+@pytest.mark.parametrize("out,inn,batch,rows", [
+    (4096, 4096, 1, False), (4096, 4096, 3, True), (4096, 4096, 8, True), (4096, 4096, 9, False), (2048, 8192, 4, True),
+    (1024, 16384, 4, False), (2304, 10944, 1, True), (2304, 10880, 1, False), (1024, 4096, 16, False)])
+def test_group_scales_route_by_size(out, inn, batch, rows):
+    """Each side of the lines between the multi-row and the SIMT kernel, against 64 bits."""
+    qd = make_layer(out, inn, seed=2, outlier_frac=0.002, qb_size=128, device=DEV)
+    qd.g.mul_(inn ** -0.5)
+    lin = EPTQLinear.from_quantized_data(qd, torch.from_numpy(TABLES["e8_d4"]).to(DEV), "e8_d4")
+    x = make_activations(batch, inn, seed=1, device=DEV)
+    lib = _lib.load()
+    lin(x)
+    before = [lib.eptq_kernel_launch_count(k) for k in range(6)]
+    y = lin(x)
+    took = [lib.eptq_kernel_launch_count(k) - b for k, b in enumerate(before)]
+    assert took == ([0, (batch + 3) // 4, 0, 0, 0, 0] if rows else [0, 0, 0, 1, 0, 0])
+    ref = x.double() @ lin.dequantize().double().T
+    assert float((y.double() - ref).abs().max() / ref.abs().max()) <= util.REL_TOL
