@@ -5,9 +5,9 @@
 // left waiting for the reconstruction:
 //
 //   tile      TM*128 tokens x 128 outputs per block (TM = 1, 2 or 4 accumulators of
-//             128 TMEM columns each).  Reconstructing a weight tile costs ~35
-//             instructions per index and is repeated for every token tile, so the
-//             token tile is made as tall as tensor memory allows (512 tokens).
+//             128 TMEM columns each).  Reconstructing a weight tile is repeated for
+//             every token tile, so the token tile is made as tall as tensor memory
+//             allows (512 tokens).
 //   warp 0    TMA producer: per 64-wide K chunk, TM bulk-tensor loads of a
 //             128-token x 64-column activation box (128-byte swizzle) into the
 //             stage's A tiles, completion counted on the stage's `full` barrier; and,
@@ -278,9 +278,8 @@ gemm_tcgen05_ws_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
                 atomicExch(p.status, EPTQ_ERR_TIMEOUT);
         }
     } else {
-        // ---------------- weight-tile producers (256 threads), then epilogue
-        // NT/8 Q rows x 64 columns per chunk over 512 threads: CPT = 2 (NT=128) or 4 (NT=256) columns each
-        // One warp per Q row, two neighbouring columns of the chunk per lane.
+        // ---------------- weight-tile producers (512 threads), then epilogue
+        // 16 Q rows x 64 columns per chunk: one warp per Q row, two neighbouring columns of the chunk per lane.
         static_assert(NT / 8 == kProducerWarps && kChunkK == 64, "one warp per Q row");
         const int qrow = warp - 2;
         const int bm = m0 + qrow;
@@ -561,19 +560,25 @@ size_t split_bytes(int M, int T, int splits) {
     return splits > 1 ? static_cast<size_t>(tile_count(M, T)) * splits * tile_tokens(T) * kOutTile * sizeof(float) : 0;
 }
 
-// K ranges per output tile.  A 4096-output layer has 32 tiles for 148 SMs; a block's time is its chunks plus about
-// twelve chunks' worth of prologue, partial sums and ticket, and two blocks on one SM take 1.4 times as long as one.
-// Bounded by the counters, by a K range of four chunks, and by 64 MiB of partial sums.  The seven linears of a 7B
-// model's layer at 100 tokens: 730 us with one range each, 390 with K ranges alone, 352 with all of this file's changes.
+// K ranges per output tile: a 4096-output layer has 32 tiles for 148 SMs.  The times below are in hundredths of what a
+// chunk takes an E8-D4 block (about 1 us; an E8 chunk 1.3), fitted to 1 to 16 ranges of eleven layers from 768 x 768 to
+// 14336 x 4096 at 17 to 512 tokens: a block's chunks and its prologue and epilogue, for each round of blocks over the SMs
+// (two blocks on one SM take 1.6 times as long as one); then once the last block's sum, which reads every token's partial
+// sums of every range (5.7 ns a token and range).  Over that set the choice is within 2 % of the fastest in the mean
+// and never more than 1 % behind one range.  Without that last term short rows at many tokens lost: 768 x 768 E8-D4 at 512
+// tokens 34.5 us in three ranges, 25.7 in one; 1024 x 4096 71.3 us in sixteen, 49.0 in four.
+// Bounded by the counters, by a K range of four chunks, and by 64 MiB of partial sums.
 int plan_splits(int kind, int M, int N, int T) {
-    const int tiles = tile_count(M, T), chunks = (N + kChunkK - 1) / kChunkK;
+    const int tiles = tile_count(M, T), chunks = (N + kChunkK - 1) / kChunkK, tokens = T < tile_tokens(T) ? T : tile_tokens(T);
     const bool shared_sm = ws_blocks(kind, tile_tokens(T) / 128) == 2;
     if (tiles >= kMaxCounters - 1) return 1;
-    int best = 1, best_cost = 0;
+    int best = 1;
+    long long best_cost = 0;
     for (int s = 1; s <= 16 && (s == 1 || chunks / s >= 4); ++s) {
         if (split_bytes(M, T, s) > (static_cast<size_t>(64) << 20)) break;
-        const int rounds = (tiles * s + kSms - 1) / kSms;
-        const int cost = rounds * ((chunks + s - 1) / s + (s > 1 ? 12 : 9)) * (shared_sm && rounds > 1 ? 7 : 10);
+        const long long rounds = (static_cast<long long>(tiles) * s + kSms - 1) / kSms;
+        const long long block = static_cast<long long>((chunks + s - 1) / s) * (kind == EPTQ_E8 ? 130 : 100) + 400 + 2 * tokens;
+        const long long cost = rounds * block * (shared_sm && rounds > 1 ? 8 : 10) + (s > 1 ? 3000 + 10 * tokens + tokens * s * 57 / 10 : 0);
         if (s == 1 || cost < best_cost) { best = s; best_cost = cost; }
     }
     return best;

@@ -21,7 +21,9 @@ TABLES = {"e8_d4": oracle.d4_table(1.75), "e8_lattice": oracle.e8_table(1.6)}
     (128, 64, 33, 0, 0.3),               # one chunk, one range
     (1024, 2056, 300, 128, 0.004),       # group scales shared by a tile
     (1024, 2056, 100, 64, 0.02),         # group scales that change inside a tile
-    (136, 520, 513, 0, 1.1),             # nothing but critical blocks
+    (136, 520, 513, 0, 1.1),             # nothing but critical blocks, reconstructed once
+    (136, 520, 512, 0, 1.1),             # the same tile by tile
+    (768, 768, 512, 0, 0.004),           # short rows at many tokens: one range
 ])
 def test_ranges_match_oracle(kind, out, inn, tokens, qb, frac):
     qd = make_layer(out, inn, seed=out + inn + tokens, outlier_frac=frac, bias=(tokens % 2 == 1), qb_size=qb or None)
@@ -63,3 +65,28 @@ def test_every_column_meets_its_own_weight(kind, tokens, one_range):
         st = lib.eptq_linear_forward(C.byref(d), x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(), ws.numel(),
                                      torch.cuda.current_stream().cuda_stream)
         assert st == 0 and torch.equal(y, W[:, cols].T)
+
+
+@pytest.mark.parametrize("kind", ["e8_d4", "e8_lattice"])
+def test_ranges_over_token_tiles(kind):
+    """Scratch that holds the partial sums but not the weight: tile by tile, K ranges, more than one token tile."""
+    import ctypes as C
+    out, inn, tokens = 1024, 32768, 700
+    lin = EPTQLinear.from_quantized_data(make_layer(out, inn, seed=8, device=DEV), torch.from_numpy(TABLES[kind]).to(DEV), kind)
+    d = lin.descriptor()
+    lib = _lib.load()
+    x = make_activations(tokens, inn, seed=9, device=DEV)
+    ref = x.double() @ lin.dequantize().double().T
+    ws = torch.zeros((1 << 20) + (64 << 20), dtype=torch.uint8, device=DEV)          # the weight alone is 64 MiB
+    ws = ws[: ws.numel() - 256]
+    before = [lib.eptq_kernel_launch_count(k) for k in range(6)]
+    ys = []
+    for _ in range(3):
+        y = torch.empty((tokens, out), dtype=torch.float16, device=DEV)
+        assert lib.eptq_linear_forward(C.byref(d), x.data_ptr(), y.data_ptr(), tokens, ws.data_ptr(), ws.numel(),
+                                       torch.cuda.current_stream().cuda_stream) == 0
+        ys.append(y)
+    assert [lib.eptq_kernel_launch_count(k) - b for k, b in enumerate(before)] == [0, 0, 0, 0, 3, 0]     # no reconstruction
+    assert float((ys[0].double() - ref).abs().max() / ref.abs().max()) <= util.REL_TOL
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
+    assert int(ws[:4096].view(torch.int32).abs().max()) == 0                         # counters left at zero, no time-out
