@@ -3,8 +3,7 @@
 // For long prefills the weight is reconstructed ONCE by dequant.cu (bit-exact fp16, the reference's
 // dequantize_layer) into scratch, and this kernel multiplies: y (T, out) = x (T, in) * W16 (out, in)^T (+ bias),
 // fp32 accumulation in tensor memory.  The fused kernel (gemm_tcgen05_ws.cu) reconstructs every weight tile once
-// per 512 tokens, which is what holds it at 40 % of the tensor peak; here both
-// operands arrive by TMA and no thread touches them.
+// per 512 tokens, which is what bounds it; here both operands arrive by TMA and no thread touches them.
 //
 //   tile      256 tokens x 256 outputs per block: two accumulators of 128 lanes x 256 TMEM columns.
 //   warp 0    TMA producer: per 64-wide K chunk two 128-token x 64-column boxes of x and two 128-output x 64-column

@@ -706,7 +706,7 @@ __global__ void __launch_bounds__(kRowsThreads, 1) gemv_rows_kernel(const __grid
         const unsigned rd = rd_addr + par * kBuf;
         par ^= 1;
         unsigned ahead[8];
-        if constexpr (KIND == EPTQ_E8) lookup(following.q, ahead);       // behind the last step: zeros, a valid index
+        if constexpr (KIND == EPTQ_E8) lookup(following.q, ahead);       // behind the last step: an earlier step's indices
         constexpr int PLANES = NB == 4 ? 1 : 2 * BT;           // column tiles: fp16 parts, then remainders
 #pragma unroll
         for (int ks = 0; ks < 2; ++ks) {                       // 16 columns: four of this lane's eight

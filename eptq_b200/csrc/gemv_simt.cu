@@ -8,8 +8,10 @@
 // scale s[m,n] = S_group[8m/qb, n] the reference has no kernel for.
 //
 // This variant covers every shape, both codebooks, group scales, N that is not
-// a multiple of 8 and any batch; it is the path for E8 (whose 1 MB table lives
-// in L2) and for layers the tensor-core GEMV does not take.
+// a multiple of 8 and any batch; it is the path for E8 layers below a million
+// indices (the 1 MB table lives in L2), for group scales where the multi-row
+// kernel is not faster (gemv_rows.cu), for tables that are no lattice multiple
+// and for N that is not a multiple of 32.
 //
 // Work split: one warp streams one Q row over one column range with 128-bit
 // loads and decodes each index once for up to BT batch rows.  Column ranges

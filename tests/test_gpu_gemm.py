@@ -1,5 +1,5 @@
-"""Prefill path (batch > 16): tcgen05 dequantise + GEMM (tile-by-tile reconstruction below 1024 tokens, one
-reconstruction into scratch followed by the dense GEMM from 1024 tokens on) against the oracle and an fp32 matmul
+"""Prefill path (batch > 16): tcgen05 dequantise + GEMM (tile-by-tile reconstruction up to 512 tokens, one
+reconstruction into scratch followed by the dense GEMM above) against the oracle and an fp32 matmul
 of the bit-exact reconstructed weight."""
 import numpy as np
 import pytest
@@ -31,7 +31,7 @@ def timeout_flag():
     (128, 64, 128, False, None), (256, 256, 128, True, None), (136, 72, 130, False, None),
     (1024, 4096, 256, False, 128), (4096, 1024, 17, True, None), (264, 2752, 300, True, 8),
     (512, 512, 2048, False, None), (2048, 512, 300, True, None), (4104, 256, 1000, False, 8),
-    (4096, 4096, 1024, True, None), (1000, 4096, 1536, False, 8),          # 1024 tokens and more: reconstruct once + dense GEMM
+    (4096, 4096, 1024, True, None), (1000, 4096, 1536, False, 8),          # above 512 tokens: reconstruct once + dense GEMM
 ])
 def test_gemm_vs_oracle(kind, radius, out_f, in_f, tokens, bias, qb):
     qd = make_layer(out_f, in_f, seed=out_f + in_f + tokens, outlier_frac=0.004, bias=bias, qb_size=qb)
